@@ -367,3 +367,150 @@ def tolerance(case: dict):
         return {"rel": 0.0125, "max": 0.99, "differ": 0.0055}
     # 2.9e-3; of the cache's codes only the new tokens' can differ (4e-3 of one token's in 1024 or more)
     return {"rel": 0.012, "differ": 2e-5}
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+NF4_VALUES = [-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635, -0.18477343022823334, -0.09105003625154495,
+              0.0, 0.07958029955625534, 0.16093020141124725, 0.24611230945587158, 0.33791524171829224, 0.44070982933044434, 0.5626170039176941,
+              0.7229568362236023, 1.0]
+
+
+def _codebook(kind: int, dev) -> torch.Tensor:
+    if kind == ffi.KV_INT8:
+        return (torch.arange(256, device=dev, dtype=torch.float64) - 127.0) / 127.0
+    if kind == ffi.KV_NF4:
+        return torch.tensor(NF4_VALUES, device=dev, dtype=torch.float64)
+    return torch.tensor([i / 16 for i in range(15)] + [1.0], device=dev, dtype=torch.float64)
+
+
+def _rounded(x: torch.Tensor, kind: int, block: int, f16: bool):
+    """(values, block maxima) of x as a cache of this kind holds them."""
+    if kind == ffi.KV_BF16:
+        return x.bfloat16().double(), None
+    flat = x.double().flatten()
+    n = flat.numel()
+    flat = torch.nn.functional.pad(flat, (0, -n % block)).view(-1, block)
+    top = flat.abs().amax(1, keepdim=True)
+    top = top.half().double() if f16 else top
+    book = _codebook(kind, x.device)
+    at = torch.bucketize(flat / torch.where(top > 0, top, 1.0), (book[1:] + book[:-1]) / 2)
+    return (book[at] * top).flatten()[:n].view(x.shape), top.flatten()
+
+
+def _stored(cache: _Cache, s: int, length: int):
+    """The first `length` tokens of sequence s as the cache's buffers hold them: (k, v) [length, heads, dim]."""
+    view, page, kvs = cache.view, cache.view.page_tokens, []
+    for i in (0, 1):
+        def rows(t, table):
+            slot = ((table[s] - t.data_ptr()) // (t.stride(0) * t.element_size()))[: (length + page - 1) // page]
+            return t[slot].flatten(0, 1)[:length]
+        codes = rows(cache.tensors[i], cache.tables[i])
+        if cache.bf16:
+            kvs.append(codes.contiguous().view(torch.bfloat16).double())
+            continue
+        if view.kind != ffi.KV_INT8:
+            codes = torch.stack((codes >> 4, codes & 15), -1).flatten(-2)  # the even element sits in the high nibble
+        top = rows(cache.tensors[2 + i], cache.tables[2 + i]).double().repeat_interleave(view.block, -1)
+        kvs.append(_codebook(view.kind, codes.device)[codes.long()] * top)
+    return kvs
+
+
+def _rotated(x: torch.Tensor, sin, cos, pos, rotary: int) -> torch.Tensor:
+    """Half-split rotation of x [rows, heads, dim]."""
+    x = x.double()
+    if sin is None:
+        return x
+    h = rotary // 2
+    s, c = sin.double()[pos.long()][:, None], cos.double()[pos.long()][:, None]
+    a, b = x[..., :h], x[..., h:rotary]
+    return torch.cat([a * c - b * s, a * s + b * c, x[..., rotary:]], -1)
+
+
+def _attend(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
+    """Causal attention of q [T, Hq, D] over k, v [L, Hkv, D], the queries at the last T positions."""
+    (t, hq, d), (l, hkv) = q.shape, k.shape[:2]
+    out = torch.empty(t, hq, d, device=q.device, dtype=torch.float64)
+    rows = max(1, (1 << 28) // (l * (hq // hkv)))
+    for h in range(hkv):
+        kh, vh, heads = k[:, h].double(), v[:, h].double(), slice(h * (hq // hkv), (h + 1) * (hq // hkv))
+        for a in range(0, t, rows):
+            b = min(t, a + rows)
+            seen = l - t + b
+            s = q[a:b, heads].double().transpose(0, 1) @ kh[:seen].T / math.sqrt(d)
+            late = torch.arange(seen, device=q.device) > (l - t + torch.arange(a, b, device=q.device))[:, None]
+            out[a:b, heads] = (s.masked_fill_(late, -math.inf).softmax(-1) @ vh[:seen]).transpose(0, 1)
+    return out
+
+
+def _delta_layer(layer, x, z, a, b, conv_state, state, carried: bool):
+    """One gated-DeltaNet layer between its projections: (y, conv state, recurrent state)."""
+    (n, t, conv), f = x.shape, torch.nn.functional
+    front = conv_state.double() if carried else torch.zeros_like(conv_state, dtype=torch.float64)
+    frames = torch.cat([front.transpose(1, 2), x.double()], 1)
+    w = layer.conv_weight.double()
+    mixed = f.silu(sum(frames[:, i:i + t] * w[:, i] for i in range(TAPS)))
+    unit = lambda u: u / u.norm(dim=-1, keepdim=True).clamp_min(1e-3)  # noqa: E731
+    q, k = (unit(u.reshape(n, t, NK, HD)).repeat_interleave(NV // NK, 2) for u in (mixed[..., :NK * HD], mixed[..., NK * HD:2 * NK * HD]))
+    q, v = q / math.sqrt(HD), mixed[..., 2 * NK * HD:].reshape(n, t, NV, HD)
+    g = layer.neg_a_exp.double() * f.softplus(a.double() + layer.dt_bias.double())
+    decay, beta = g.exp(), torch.sigmoid(b.double())
+    s, out = (state.double().clone() if carried else torch.zeros_like(state, dtype=torch.float64)), torch.empty_like(v)
+    for i in range(t):
+        s *= decay[:, i, :, None, None]
+        ki = k[:, i, :, None, :]
+        s += ki.transpose(-1, -2) * ((v[:, i, :, None, :] - ki @ s) * beta[:, i, :, None, None])
+        out[:, i] = (q[:, i, :, None, :] @ s)[:, :, 0]
+    norm = out * torch.rsqrt(out.square().mean(-1, keepdim=True) + 1e-6)
+    return norm * layer.norm_weight.double() * f.silu(z.double()), frames[:, t:].transpose(1, 2).contiguous(), s
+
+
+def exact(case: dict, seed: int):
+    """What `run` returns, worked out in 64 bits; None for caches (their codes and block maxima are roundings of the inputs)."""
+    st, w = prepare(case, seed), case["work"]
+    if w == "tensor":
+        values, top = _rounded(st["x"], st["kind"], st["block"], case["f16"])
+        return [None, top, values]
+    if w in ("qstep", "qprompt"):
+        b, t, attn = st["b"], st["t"], st["attn"]
+        if t * b > 70000:
+            return None  # the recurrence takes too long one token at a time
+        layers = [_delta_layer(l, *g, st["has"]) for l, g in zip(st["layers"], st["gin"])]
+        qp, kp, v, _, pos, _, lens = st["ain"]
+
+        def normed(x, weight):
+            x = x.double()
+            return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * (1.0 + weight.double())
+        qg = qp.view(b * t, QHQ, 2 * QD)
+        q = _rotated(normed(qg[..., :QD], attn.qw), attn.sin, attn.cos, pos, QROT).view(b, t, QHQ, QD)
+        k = _rotated(normed(kp.view(b * t, QHKV, QD), attn.kw), attn.sin, attn.cos, pos, QROT).view(b, t, QHKV, QD)
+        out = torch.empty(b, t, QHQ, QD, device=st["dev"], dtype=torch.float64)
+        for s in range(b):
+            ks, vs = k[s], v[s]
+            if w == "qstep":
+                old = _stored(st["cache"], s, int(lens[s]) - 1)
+                ks, vs = (torch.cat([o, _rounded(x, ffi.KV_INT8, case["block"], case["f16"])[0]]) for o, x in zip(old, (ks, vs)))
+            out[s] = _attend(q[s], ks, vs)
+        out *= torch.sigmoid(qg[..., QD:].double().view(b, t, QHQ, QD))
+        return [l[0] for l in layers] + [out] + [s for l in layers for s in l[1:]] + [None] * len(st["cache"].tensors)
+    if w == "chunk":
+        rnd, p, t, hkv, d = _Gen(seed), case["prefix"], case["t"], case["hkv"], case["d"]
+        old = [rnd.b(1, p, hkv, d) for _ in range(2)]
+        k, v = (_rounded(torch.cat([o, st[x]], 1), KINDS[case["kind"]], case["block"], case["f16"])[0] for o, x in zip(old, "kv"))
+        return [_attend(st["q"][0], k[0], v[0])[None], k, v]
+    cache, hkv, d, n = st["cache"], case["hkv"], case["d"], case["n"]
+    none = [None] * len(cache.tensors)
+    if w == "prompt":
+        t = st["t"]
+        q, k = (_rotated(st[x], st["sin"], st["cos"], st["pos"], st["rotary"]).view(n, t, -1, d) for x in "qk")
+        return [torch.stack([_attend(q[s], k[s], st["v"][s]) for s in range(n)])] + none
+    lens = st["lens"]
+    q, k, v = (getattr(st["step"], x + "_host").to(lens.device) for x in "qkv") if w == "hoststep" else (st["q"], st["k"], st["v"])
+    if w == "step":
+        q = _rotated(q, st["sin"], st["cos"], lens - 1, st["rotary"])
+    k = _rotated(k.reshape(n, hkv, d), st["sin"], st["cos"], lens - 1, st["rotary"])
+    out = []
+    for s in range(n):
+        old, new = _stored(cache, s, int(lens[s]) - 1), (k[s:s + 1], v.reshape(n, 1, hkv, d)[s])
+        ks, vs = (torch.cat([o, _rounded(x, KINDS[case["kind"]], case["block"], case["f16"])[0]]) for o, x in zip(old, new))
+        out.append(_attend(q[s:s + 1], ks, vs))
+    return [torch.cat(out)] + none
