@@ -6,8 +6,8 @@
 // llama.rs:710-844 with its padding mask 2540-2572; qwen3_5.rs:992-1059 for the gated variant).
 // The cache is read exactly once, in its stored precision, and dequantised in registers.
 //
-// This file holds the shape-generic CUDA-core kernel (any supported kind, head_dim 64/128/256,
-// group 1/2/4/8) and the merge kernel.  It is HBM-bound: per cached token and kv head it moves
+// This file holds the shape-generic CUDA-core kernel (quantised kinds, head_dim 64/128/256, group 1/2/4/8; a bf16 cache
+// goes to decode_mma.cu) and the merge kernel.  It is HBM-bound: per cached token and kv head it moves
 // 2*head_dim code bytes plus the scales, and does 2*group*head_dim FMAs.
 #include <mutex>
 
@@ -25,26 +25,19 @@ __device__ __forceinline__ int ceil_div_i(int a, int b) { return (a + b - 1) / b
 // Raw (unscaled) values of EPL consecutive elements starting at element `e` of a page.
 template <int KIND, int EPL>
 struct Chunk {
-    static constexpr int kWords = KIND == HS_KV_BF16 ? EPL / 2 : (KIND == HS_KV_INT8 ? EPL / 4 : EPL / 8);
+    static constexpr int kWords = KIND == HS_KV_INT8 ? EPL / 4 : EPL / 8;
     uint32_t w[kWords];
 
     __device__ __forceinline__ void load(const void *page, int64_t e) {
-        if constexpr (kWords == 8) {
-            const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(page) + e);
-            uint4 a = p[0], b = p[1];
-            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+        const char *base = reinterpret_cast<const char *>(page) + (KIND == HS_KV_INT8 ? e : e / 2);
+        if constexpr (kWords == 4) {
+            uint4 a = *reinterpret_cast<const uint4 *>(base);
+            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        } else if constexpr (kWords == 2) {
+            uint2 a = *reinterpret_cast<const uint2 *>(base);
+            w[0] = a.x; w[1] = a.y;
         } else {
-            const char *base = reinterpret_cast<const char *>(page) +
-                               (KIND == HS_KV_BF16 ? e * 2 : (KIND == HS_KV_INT8 ? e : e / 2));
-            if constexpr (kWords == 4) {
-                uint4 a = *reinterpret_cast<const uint4 *>(base);
-                w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-            } else if constexpr (kWords == 2) {
-                uint2 a = *reinterpret_cast<const uint2 *>(base);
-                w[0] = a.x; w[1] = a.y;
-            } else {
-                w[0] = *reinterpret_cast<const uint32_t *>(base);
-            }
+            w[0] = *reinterpret_cast<const uint32_t *>(base);
         }
     }
     __device__ __forceinline__ void zero() {
@@ -53,9 +46,7 @@ struct Chunk {
     }
     // element i as a float before the block scale is applied (int8: code - 127; 4-bit: table value)
     __device__ __forceinline__ float get(int i, const float *stab) const {
-        if constexpr (KIND == HS_KV_BF16) {
-            return (i & 1) ? bf16hi(w[i >> 1]) : bf16lo(w[i >> 1]);
-        } else if constexpr (KIND == HS_KV_INT8) {
+        if constexpr (KIND == HS_KV_INT8) {
             // 2^23 + byte, built with one byte permute, minus (2^23 + 127): exact
             return __uint_as_float(__byte_perm(w[i >> 2], 0x4B000000u, 0x7650 + (i & 3))) - 8388735.0f;
         } else {
@@ -132,8 +123,8 @@ decode_generic_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_
         }
         void *const *kp = view.k_pages + static_cast<int64_t>(r) * view.pages_per_seq;
         void *const *vp = view.v_pages + static_cast<int64_t>(r) * view.pages_per_seq;
-        void *const *ksp = KIND == HS_KV_BF16 ? nullptr : view.k_scale_pages + static_cast<int64_t>(r) * view.pages_per_seq;
-        void *const *vsp = KIND == HS_KV_BF16 ? nullptr : view.v_scale_pages + static_cast<int64_t>(r) * view.pages_per_seq;
+        void *const *ksp = view.k_scale_pages + static_cast<int64_t>(r) * view.pages_per_seq;
+        void *const *vsp = view.v_scale_pages + static_cast<int64_t>(r) * view.pages_per_seq;
 
         for (int tb = tok_begin; tb < tok_end; tb += NG * U) {  // warp-uniform trip count
             Chunk<KIND, EPL> kc[U], vc[U];
@@ -149,10 +140,8 @@ decode_generic_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_
                     const int64_t row = static_cast<int64_t>(t - page * view.page_tokens) * H + kvh;
                     kc[u].load(kp[page], row * D + d0);
                     vc[u].load(vp[page], row * D + d0);
-                    if constexpr (KIND != HS_KV_BF16) {
-                        ks[u] = load_scale(ksp[page], row * bpr + sblk, view.scale_dtype) * kscale_mul;
-                        vs[u] = load_scale(vsp[page], row * bpr + sblk, view.scale_dtype) * kscale_mul;
-                    }
+                    ks[u] = load_scale(ksp[page], row * bpr + sblk, view.scale_dtype) * kscale_mul;
+                    vs[u] = load_scale(vsp[page], row * bpr + sblk, view.scale_dtype) * kscale_mul;
                 } else {
                     kc[u].zero(); vc[u].zero();
                 }
@@ -229,96 +218,86 @@ decode_generic_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_
     }
 }
 
-// Merge the split-KV partials of one sequence, kMergeHeads query heads per CTA.  The slot range of the
-// sequence is recomputed from seq_lens with the same partition arithmetic the decode kernel used: CTA c
-// and sequence r share slots (c + r) * ppp + k, k < ppp (ppp = partials each pair writes).
+// Merge the split-KV partials of one (sequence, query head) per CTA.  The CTAs that hold tiles of the sequence follow from
+// seq_lens with the same partition arithmetic the decode kernel used: CTA c and sequence r share slot c + r, no CTA of the
+// range is empty, so the partials are consecutive.  Latency bound (a few dozen partials of D floats from L2): D / 4 threads
+// take a partial with 16-byte loads and the CTA's thread groups take every kMergeThreads / (D / 4)-th, so that a batch of one
+// sequence has all its partials in flight at once.  One query head a CTA and closed-form ends of the range instead of four
+// heads a CTA and one thread walking the CTA list with 64-bit divisions: 50.8 -> 8.2 us for 1 x 4096 tokens (a cold launch by itself).
 constexpr int kMergeThreads = 256;
-constexpr int kMergeHeads = 4;
-constexpr int kMergeMaxParts = 1280;  // >= decode_max_ctas() * kMaxPartsPerPair on a 148-SM part (checked on the host)
 __global__ void __launch_bounds__(kMergeThreads)
 decode_merge_kernel(const int32_t *__restrict__ seq_lens, int n_seqs, int n_q_heads, int D, int n_ctas, int tile, int cap,
-                    int ppp, const float *__restrict__ o_part, const float *__restrict__ lse_part, uint16_t *__restrict__ out,
+                    const float *__restrict__ o_part, const float *__restrict__ lse_part, uint16_t *__restrict__ out,
                     const uint16_t *__restrict__ gate, float *__restrict__ o_shard, float *__restrict__ lse_shard) {
-    __shared__ int s_slot[kMergeMaxParts];
-    __shared__ float s_w[kMergeMaxParts * kMergeHeads];
-    __shared__ float s_den[kMergeHeads], s_max[kMergeHeads];
-    __shared__ int s_nparts;
-    const int r = blockIdx.x, h0 = blockIdx.y * kMergeHeads, lane = threadIdx.x & 31;
-    const int nh = min(kMergeHeads, n_q_heads - h0);
+    __shared__ float4 s_num[kMergeThreads];
+    const int r = blockIdx.x / n_q_heads, h = blockIdx.x - r * n_q_heads, lane = threadIdx.x & 31;
     // every warp computes the tile prefix redundantly, one coalesced load per 32 sequences
-    long long total = 0, before = 0;
+    int64_t total = 0, before = 0;
     for (int base = 0; base < n_seqs; base += 32) {
         const int i = base + lane;
-        const int t = i < n_seqs ? ceil_div_i(min(max(seq_lens[i], 0), cap), tile) : 0;
-        total += t;
-        before += i < r ? t : 0;
+        const unsigned t = i < n_seqs ? ceil_div_i(min(max(seq_lens[i], 0), cap), tile) : 0;
+        total += __reduce_add_sync(0xffffffffu, t);
+        before += __reduce_add_sync(0xffffffffu, i < r ? t : 0u);
+    }
+    const int64_t nt = ceil_div_i(min(max(seq_lens[r], 0), cap), tile);
+    if (total < n_ctas) n_ctas = total > 0 ? static_cast<int>(total) : 1;  // the decode kernels never use more CTAs than tiles
+    int np = 0;
+    int64_t slot0 = 0;
+    if (nt > 0) {
+        // tile t belongs to the last CTA c with floor(c * total / n_ctas) <= t, i.e. c * total < (t + 1) * n_ctas
+        const int64_t c_lo = ((before + 1) * n_ctas - 1) / total, c_hi = ((before + nt) * n_ctas - 1) / total;
+        np = static_cast<int>(c_hi - c_lo + 1);
+        slot0 = c_lo + r;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // everything above overlaps with the decode kernel's end; its partials are read below
+    const float *lse = lse_part + slot0 * n_q_heads + h;
+    float M = -INFINITY;
+    for (int i = lane; i < np; i += 32) M = fmaxf(M, lse[static_cast<int64_t>(i) * n_q_heads]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+    float den = 0.0f;
+    for (int i = lane; i < np; i += 32) {
+        const float ls = lse[static_cast<int64_t>(i) * n_q_heads];
+        den += ls == -INFINITY ? 0.0f : __expf(ls - M);
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        total += __shfl_xor_sync(0xffffffffu, total, off);
-        before += __shfl_xor_sync(0xffffffffu, before, off);
+    for (int off = 16; off > 0; off >>= 1) den += __shfl_xor_sync(0xffffffffu, den, off);
+    const int dt = D / 4, groups = kMergeThreads / dt;          // threads per partial, partials at a time
+    const int grp = threadIdx.x / dt, d = (threadIdx.x - grp * dt) * 4;
+    const float *op = o_part + (slot0 * n_q_heads + h) * D + d;
+    const int64_t stride = static_cast<int64_t>(n_q_heads) * D;
+    float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int i = grp; i < np; i += groups) {
+        const float ls = lse[static_cast<int64_t>(i) * n_q_heads];
+        const float4 v = *reinterpret_cast<const float4 *>(op + i * stride);
+        const float w = ls == -INFINITY ? 0.0f : __expf(ls - M);
+        num.x = fmaf(w, v.x, num.x); num.y = fmaf(w, v.y, num.y); num.z = fmaf(w, v.z, num.z); num.w = fmaf(w, v.w, num.w);
     }
-    const long long nt = ceil_div_i(min(max(seq_lens[r], 0), cap), tile);
-    if (total < n_ctas) n_ctas = total > 0 ? static_cast<int>(total) : 1;  // the decode kernels never use more CTAs than tiles
-    if (threadIdx.x == 0) {
-        // CTAs whose tile range overlaps [before, before + nt); a CTA with an empty range wrote nothing
-        int n = 0;
-        if (nt > 0) {
-            long long c = before * n_ctas / total;
-            while (c > 0 && part_begin(c, total, n_ctas) > before) --c;
-            while (part_begin(c + 1, total, n_ctas) <= before) ++c;
-            for (; c < n_ctas && part_begin(c, total, n_ctas) < before + nt; ++c) {
-                if (part_begin(c, total, n_ctas) >= part_begin(c + 1, total, n_ctas)) continue;
-                for (int k = 0; k < ppp && n < kMergeMaxParts; ++k) s_slot[n++] = static_cast<int>((c + r) * ppp + k);
-            }
-        }
-        s_nparts = n;
-    }
+    s_num[threadIdx.x] = num;
     __syncthreads();
-    const int np = s_nparts;
-    for (int i = threadIdx.x; i < np * nh; i += kMergeThreads) {
-        const int pi = i / nh, hh = i - pi * nh;
-        s_w[pi * kMergeHeads + hh] = lse_part[static_cast<int64_t>(s_slot[pi]) * n_q_heads + h0 + hh];
+    if (grp != 0) return;
+    for (int k = 1; k < groups; ++k) {
+        const float4 v = s_num[k * dt + threadIdx.x];
+        num.x += v.x; num.y += v.y; num.z += v.z; num.w += v.w;
     }
-    __syncthreads();
-    if (threadIdx.x < nh) {
-        float M = -INFINITY;
-        for (int pi = 0; pi < np; ++pi) M = fmaxf(M, s_w[pi * kMergeHeads + threadIdx.x]);
-        s_max[threadIdx.x] = M;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < np * nh; i += kMergeThreads) {
-        const int pi = i / nh, hh = i - pi * nh;
-        const float ls = s_w[pi * kMergeHeads + hh];
-        s_w[pi * kMergeHeads + hh] = ls == -INFINITY ? 0.0f : __expf(ls - s_max[hh]);
-    }
-    __syncthreads();
-    if (threadIdx.x < nh) {
-        float den = 0.0f;
-        for (int pi = 0; pi < np; ++pi) den += s_w[pi * kMergeHeads + threadIdx.x];
-        s_den[threadIdx.x] = den;
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < nh * D; idx += kMergeThreads) {
-        const int hh = idx / D, d = idx - hh * D;
-        const int64_t row = static_cast<int64_t>(r) * n_q_heads + h0 + hh;
-        float num = 0.0f;
-        for (int pi = 0; pi < np; ++pi)
-            num = fmaf(s_w[pi * kMergeHeads + hh], o_part[(static_cast<int64_t>(s_slot[pi]) * n_q_heads + h0 + hh) * D + d], num);
-        const float den = s_den[hh];
-        const float o = den > 0.0f ? num / den : 0.0f;
+    const int64_t row = static_cast<int64_t>(r) * n_q_heads + h;
+    const float o[4] = {num.x, num.y, num.z, num.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float v = den > 0.0f ? o[i] / den : 0.0f;
         if (o_shard != nullptr) {
-            o_shard[row * D + d] = o;
-            if (d == 0) lse_shard[row] = den > 0.0f ? s_max[hh] + __logf(den) : -INFINITY;
+            o_shard[row * D + d + i] = v;
             continue;
         }
-        float res = o;
+        float res = v;
         if (gate != nullptr) {
-            const float gv = bf16_bits_to_f32(gate[row * D + d]);
-            res = bf16_round(o) * bf16_round(1.0f / (1.0f + __expf(-gv)));  // ctx * sigmoid(gate) in bf16 (qwen3_5.rs:1056-1059)
+            const float gv = bf16_bits_to_f32(gate[row * D + d + i]);
+            res = bf16_round(v) * bf16_round(1.0f / (1.0f + __expf(-gv)));  // ctx * sigmoid(gate) in bf16 (qwen3_5.rs:1056-1059)
         }
-        out[row * D + d] = f32_to_bf16_bits(res);
+        out[row * D + d + i] = f32_to_bf16_bits(res);
     }
+    if (o_shard != nullptr && d == 0) lse_shard[row] = den > 0.0f ? M + __logf(den) : -INFINITY;
 }
 
 // Merge of externally produced partials (KV-length shards from several GPUs, or a caller's own split).
@@ -353,6 +332,10 @@ int32_t decode_int8_tc_try(const ViewDev &v, const uint16_t *q, const int32_t *s
                            float softmax_scale, float *o_part, float *lse_part, int *err, cudaStream_t s, int *n_ctas_out,
                            uint16_t *out, const uint16_t *gate, float *o_shard, float *lse_shard, int *merged_out,
                            const ShardArgs *shard, int after_write, const AppendArgs *append);
+
+// decode_mma.cu: tensor-core kernel for bf16 caches of every supported shape
+int32_t decode_bf16_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
+                        float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, cudaStream_t s);
 
 template <int KIND, int D, int G>
 static int32_t launch_generic(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads,
@@ -486,7 +469,7 @@ int32_t hs::decode_impl(const void *q, const hs_kv_view *view, const int32_t *se
     cudaStream_t s = as_stream(stream);
     const uint16_t *qp = reinterpret_cast<const uint16_t *>(q);
     int32_t st;
-    int tile = kDecTile, tc_ctas = 0, ppp = 1, merged = 0;
+    int tile = kDecTile, tc_ctas = 0, merged = 0;
     prof_begin(s);
     st = decode_int8_tc_try(v, qp, seq_lens, n_seqs, n_q_heads, softmax_scale, o_part, lse_part, err, s, &tc_ctas,
                             reinterpret_cast<uint16_t *>(out), reinterpret_cast<const uint16_t *>(gate), o_shard, lse_shard, &merged, shard, after_write, append);
@@ -501,12 +484,11 @@ int32_t hs::decode_impl(const void *q, const hs_kv_view *view, const int32_t *se
                                         "with 32 query heads or 2 x 256 with 16, cooperative launch available); use hs_attn_decode with o_shard / lse_shard, an "
                                         "all-gather and hs_attn_merge_partials_strided for this shape");
     }
-    if (st == HS_OK && tc_ctas > 0) {
-        n_ctas = tc_ctas;
-        tile = 16;
-    } else if (st == HS_OK) {
+    if (st == HS_OK && tc_ctas == 0) {
         switch (view->kind) {
-            case HS_KV_BF16: st = dispatch_d<HS_KV_BF16>(D, G, v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, n_ctas, s); break;
+            case HS_KV_BF16:
+                st = decode_bf16_mma(v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, decode_max_ctas(), &n_ctas, &tile, after_write != 0, s);
+                break;
             case HS_KV_INT8: st = dispatch_d<HS_KV_INT8>(D, G, v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, n_ctas, s); break;
             default: st = dispatch_d<kKind4Bit>(D, G, v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, n_ctas, s); break;
         }
@@ -515,11 +497,23 @@ int32_t hs::decode_impl(const void *q, const hs_kv_view *view, const int32_t *se
     if (st != HS_OK) return st;
     if (int32_t e = check_launch("hs_attn_decode")) return e;
     if (merged) return HS_OK;  // the decode kernel merged its own partials behind a grid barrier
-    if (static_cast<int64_t>(n_ctas) * ppp > kMergeMaxParts) return fail(HS_ERR_UNSUPPORTED, "hs_attn_decode: %d partial slots exceed the merge kernel's table", n_ctas * ppp);
-    dim3 mgrid(n_seqs, (n_q_heads + kMergeHeads - 1) / kMergeHeads);
-    decode_merge_kernel<<<mgrid, kMergeThreads, 0, s>>>(seq_lens, n_seqs, n_q_heads, D, n_ctas, tile, v.page_tokens * v.pages_per_seq, ppp, o_part,
-                                            lse_part, reinterpret_cast<uint16_t *>(out), reinterpret_cast<const uint16_t *>(gate),
-                                            o_shard, lse_shard);
+    // the merge is launched as the decode kernel's programmatic dependent: its launch and its slot arithmetic overlap with it
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(n_seqs) * static_cast<unsigned>(n_q_heads));
+    cfg.blockDim = dim3(kMergeThreads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t me = cudaLaunchKernelEx(&cfg, decode_merge_kernel, seq_lens, static_cast<int>(n_seqs), static_cast<int>(n_q_heads), D, n_ctas, tile,
+                                              v.page_tokens * v.pages_per_seq, static_cast<const float *>(o_part), static_cast<const float *>(lse_part),
+                                              reinterpret_cast<uint16_t *>(out), reinterpret_cast<const uint16_t *>(gate), o_shard, lse_shard);
+    if (me != cudaSuccess) {
+        cudaGetLastError();
+        return fail(static_cast<int32_t>(me), "hs_attn_decode (merge): %s", cudaGetErrorString(me));
+    }
     return check_launch("hs_attn_decode (merge)");
 }
 
