@@ -406,8 +406,8 @@ decode_int8_tc_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_
                 float x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
                 const uint16_t *src = (is_v ? mg.append.v_new : mg.append.k_new) + (static_cast<int64_t>(r) * H + hh) * kD;
                 if (okw) load_row8_rope(src, d0, rope ? mg.append.sin : nullptr, mg.append.cos, pos, mg.append.rotary_dim, x);
-                int c[8];
-                const float a = quantize_n<HS_KV_INT8, 8>(x, tpb, view.scale_dtype, nullptr, c);  // (every lane takes part in the shuffles)
+                CodeWords<HS_KV_INT8, 8> c;
+                const float a = quantize_n<HS_KV_INT8, 8>(x, tpb, view.scale_dtype, IndexDirect{}, c);  // (every lane takes part in the shuffles)
                 if (!okw) continue;
                 const int64_t pidx = static_cast<int64_t>(r) * view.pages_per_seq + page;
                 const int64_t in_page = static_cast<int64_t>(pos - page * view.page_tokens) * H + hh;

@@ -10,93 +10,186 @@
 // Codebooks and block geometry follow bitsandbytes-sys/src/lib.rs:104-181 and
 // crates/hyprstream/src/runtime/kv_cache.rs:704,741-957.
 //
-// All kernels here are HBM-streaming: one thread owns 8 consecutive elements (one 16-byte bf16
-// load, one 8-byte int8 store), a block's absmax is reduced with warp shuffles, nothing is staged.
+// All kernels here are HBM-streaming: a thread owns chunks of 8 (16) consecutive elements with 16-byte loads and stores,
+// a block's absmax is reduced with warp shuffles, nothing is staged.
 #include "hs_common.cuh"
 #include "quant_dev.cuh"
 
 namespace hs {
 
 constexpr int kQThreads = 256;
-#ifndef HS_KV_WRITE_WIDE
-#define HS_KV_WRITE_WIDE 16
-#endif
 constexpr int kWriteElems = 64;  // elements per thread of the quantise-on-write kernel (as 8- or 16-element chunks)
 
 // ---- flat quantise ----------------------------------------------------------------------------
-template <int KIND>
-__global__ void __launch_bounds__(kQThreads) quantize_flat_kernel(const void *__restrict__ src, int dtype, int64_t n,
-                                                                  int block, int scale_dtype, uint8_t *__restrict__ codes,
-                                                                  void *__restrict__ absmax, int vec_ok) {
-    __shared__ float smid[256];
-    fill_midpoints(KIND, smid);
-    __syncthreads();
-    const int64_t chunk = static_cast<int64_t>(blockIdx.x) * kQThreads + threadIdx.x;
-    const int64_t e0 = chunk * 8;
-    float x[8];
-    const bool full = e0 + 8 <= n;
-    if (full && vec_ok && dtype == HS_DTYPE_BF16) {
-        unpack8_bf16(*reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(src) + e0), x);
+// HBM streaming by design.  A thread takes kFlatChunks chunks of 8 elements, all of them loaded before the first is worked on
+// (one chunk per thread left too few bytes in flight), 16-byte loads for every dtype, and a 4-bit index is one lookup instead
+// of 15 comparisons (quant_dev.cuh).
+constexpr int kFlatChunks = 4;
+
+template <int DTYPE>
+__device__ __forceinline__ void load_chunk8(const void *src, int64_t e0, int64_t n, bool vec, float (&x)[8]) {
+    if (vec && e0 + 8 <= n) {
+        if constexpr (DTYPE == HS_DTYPE_F32) {
+            const float4 *p = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(src) + e0);
+            const float4 a = p[0], b = p[1];
+            x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+        } else {
+            const uint4 w = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(src) + e0);
+            if constexpr (DTYPE == HS_DTYPE_BF16) {
+                unpack8_bf16(w, x);
+            } else {
+                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&ww[i]));
+                    x[2 * i] = f.x; x[2 * i + 1] = f.y;
+                }
+            }
+        }
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = (e0 + i < n) ? load_elem(src, dtype, e0 + i) : 0.0f;
+        for (int i = 0; i < 8; ++i) x[i] = (e0 + i < n) ? load_elem(src, DTYPE, e0 + i) : 0.0f;
     }
-    int c[8];
-    const int tpb = block / 8;
-    float a = quantize8<KIND>(x, tpb, scale_dtype, smid, c);
-    if (e0 < n) {
-        if ((chunk % tpb) == 0) store_scale(absmax, e0 / block, scale_dtype, a);
-        store_codes8<KIND>(codes, e0, n, c, full);
+}
+
+template <int KIND, int DTYPE>
+__global__ void __launch_bounds__(kQThreads) quantize_flat_kernel(const void *__restrict__ src, int64_t n,
+                                                                  int block, int scale_dtype, uint8_t *__restrict__ codes,
+                                                                  void *__restrict__ absmax, int vec_ok) {
+    __shared__ IndexTable<KIND> tab;
+    tab.fill();
+    __syncthreads();
+    const int64_t chunk0 = static_cast<int64_t>(blockIdx.x) * (kQThreads * kFlatChunks) + threadIdx.x;
+    const int tpb = block / 8, block_shift = __ffs(block) - 1;
+    float x[kFlatChunks][8];
+#pragma unroll
+    for (int u = 0; u < kFlatChunks; ++u) load_chunk8<DTYPE>(src, (chunk0 + u * kQThreads) * 8, n, vec_ok != 0, x[u]);
+#pragma unroll
+    for (int u = 0; u < kFlatChunks; ++u) {
+        const int64_t chunk = chunk0 + u * kQThreads, e0 = chunk * 8;
+        CodeWords<KIND, 8> c;
+        const float a = quantize_n<KIND, 8>(x[u], tpb, scale_dtype, tab, c);
+        if (e0 < n) {
+            if ((threadIdx.x & (tpb - 1)) == 0) store_scale(absmax, e0 >> block_shift, scale_dtype, a);
+            store_codes8<KIND>(codes, e0, n, c, e0 + 8 <= n);
+        }
     }
 }
 
 // ---- flat dequantise ----------------------------------------------------------------------------
-__device__ __forceinline__ float table_value(int kind, int c, const float *stab) {
-    return kind == HS_KV_INT8 ? code8(c) : stab[c];
-}
-
 __device__ __forceinline__ void store_elem(void *out, int dtype, int64_t i, float v) {
     if (dtype == HS_DTYPE_BF16) reinterpret_cast<uint16_t *>(out)[i] = f32_to_bf16_bits(v);
     else if (dtype == HS_DTYPE_F16) reinterpret_cast<__half *>(out)[i] = __float2half_rn(v);
     else reinterpret_cast<float *>(out)[i] = v;
 }
 
-__global__ void __launch_bounds__(kQThreads) dequantize_flat_kernel(int kind, const uint8_t *__restrict__ codes,
+// A thread takes kFlatChunks chunks of 8 elements: whole-word loads of the codes, 16-byte stores (element-wise only at the end
+// of the tensor and for buffers that are not aligned for it).  The 8-bit codebook is worked out ((code - 127) / 127, one IEEE
+// division: a 256-entry table in shared memory), the 4-bit ones are looked up in a table that every lane has a column of.
+template <int KIND, int DTYPE>
+__global__ void __launch_bounds__(kQThreads) dequantize_flat_kernel(const uint8_t *__restrict__ codes,
                                                                     const void *__restrict__ absmax, int64_t n, int block,
-                                                                    int scale_dtype, void *__restrict__ out, int dtype) {
-    __shared__ float stab[16];
-    if (kind != HS_KV_INT8 && threadIdx.x < 16) stab[threadIdx.x] = kind == HS_KV_NF4 ? c_nf4[threadIdx.x] : c_fp4[threadIdx.x];
+                                                                    int scale_dtype, void *__restrict__ out, int vec_ok) {
+    __shared__ ValueTable<KIND> tab;
+    tab.fill();
     __syncthreads();
-    const int64_t e0 = (static_cast<int64_t>(blockIdx.x) * kQThreads + threadIdx.x) * 8;
-    if (e0 >= n) return;
-    const float a = load_scale(absmax, e0 / block, scale_dtype);
-    for (int i = 0; i < 8 && e0 + i < n; ++i) {
-        int64_t e = e0 + i;
-        int c = kind == HS_KV_INT8 ? codes[e] : ((e & 1) ? (codes[e >> 1] & 0xf) : (codes[e >> 1] >> 4));
-        store_elem(out, dtype, e, __fmul_rn(table_value(kind, c, stab), a));
+    const int64_t chunk0 = static_cast<int64_t>(blockIdx.x) * (kQThreads * kFlatChunks) + threadIdx.x;
+    const bool pow2 = (block & (block - 1)) == 0;
+    const int block_shift = __ffs(block) - 1;
+    uint2 w[kFlatChunks];
+    float a[kFlatChunks];
+#pragma unroll
+    for (int u = 0; u < kFlatChunks; ++u) {
+        const int64_t e0 = (chunk0 + u * kQThreads) * 8;
+        w[u] = make_uint2(0u, 0u);
+        a[u] = 0.0f;
+        if (e0 < n) {
+            a[u] = load_scale(absmax, pow2 ? e0 >> block_shift : e0 / block, scale_dtype);
+            if (vec_ok && e0 + 8 <= n) {
+                if constexpr (KIND == HS_KV_INT8) w[u] = *reinterpret_cast<const uint2 *>(codes + e0);
+                else w[u].x = *reinterpret_cast<const uint32_t *>(codes + (e0 >> 1));
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kFlatChunks; ++u) {
+        const int64_t e0 = (chunk0 + u * kQThreads) * 8;
+        if (e0 >= n) return;
+        if (vec_ok && e0 + 8 <= n) {
+            float v[8];
+            tab.values8(w[u], v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(v[i], a[u]);
+            if constexpr (DTYPE == HS_DTYPE_F32) {
+                float4 *p = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + e0);
+                p[0] = make_float4(v[0], v[1], v[2], v[3]);
+                p[1] = make_float4(v[4], v[5], v[6], v[7]);
+            } else {
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if constexpr (DTYPE == HS_DTYPE_BF16) {
+                        o[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+                    } else {
+                        const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+                        o[i] = *reinterpret_cast<const uint32_t *>(&h);
+                    }
+                }
+                *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(out) + e0) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        } else {
+            for (int i = 0; i < 8 && e0 + i < n; ++i) {
+                const int64_t e = e0 + i;
+                const int c = KIND == HS_KV_INT8 ? codes[e] : ((e & 1) ? (codes[e >> 1] & 0xf) : (codes[e >> 1] >> 4));
+                store_elem(out, DTYPE, e, __fmul_rn(tab.value(c), a[u]));
+            }
+        }
     }
 }
 
 // ---- RoPE (device helpers in quant_dev.cuh) ------------------------------------------------------------
+// A thread takes the 8 elements at j of a head's first rotated half together with their partners in the second half - both are
+// read and written once, and one pair of sin / cos loads serves both - or 8 elements that pass through unrotated.  HBM bound: a
+// block covers whole rows (one position each) with 32-bit arithmetic; the 64-bit divisions per 8 elements of the earlier form
+// were most of its instructions.
 __global__ void __launch_bounds__(kQThreads) rope_kernel(const uint16_t *__restrict__ x, uint16_t *__restrict__ out,
                                                          const uint16_t *__restrict__ sin, const uint16_t *__restrict__ cos,
                                                          const int32_t *__restrict__ positions, int64_t n_rows, int n_heads,
-                                                         int head_dim, int rotary_dim, int n_positions, int *__restrict__ err) {
-    const int cpr = head_dim / 8;  // chunks per (row, head)
-    const int64_t chunk = static_cast<int64_t>(blockIdx.x) * kQThreads + threadIdx.x;
-    const int64_t total = n_rows * n_heads * cpr;
-    if (chunk >= total) return;
-    const int d0 = static_cast<int>(chunk % cpr) * 8;
-    const int64_t rh = chunk / cpr;
-    const int64_t r = rh / n_heads;
-    float v[8];
-    const int pos = positions[r];
-    const bool in_table = pos >= 0 && pos < n_positions;
-    if (!in_table) atomicOr(err, HS_DEVERR_ROPE_RANGE);  // recorded; the row is copied unrotated
-    load_row8_rope(x + rh * head_dim, d0, in_table ? sin : nullptr, cos, in_table ? pos : 0, rotary_dim, v);
-    uint4 w;
-    w.x = pack_bf16(v[0], v[1]); w.y = pack_bf16(v[2], v[3]); w.z = pack_bf16(v[4], v[5]); w.w = pack_bf16(v[6], v[7]);
-    *reinterpret_cast<uint4 *>(out + rh * head_dim + d0) = w;
+                                                         int head_dim, int rotary_dim, int n_positions, int rows_per_block, int *__restrict__ err) {
+    const int half = rotary_dim >> 1;
+    const unsigned rot = static_cast<unsigned>(half) / 8u;                               // rotated pairs of chunks per head
+    const unsigned upr = rot + static_cast<unsigned>(head_dim - rotary_dim) / 8u;        // work units per head
+    const unsigned units = upr * static_cast<unsigned>(n_heads);                         // ... and per row
+    const int64_t row0 = static_cast<int64_t>(blockIdx.x) * rows_per_block;
+    const unsigned rows = static_cast<unsigned>(min(static_cast<int64_t>(rows_per_block), n_rows - row0));
+#pragma unroll 2
+    for (unsigned i = threadIdx.x; i < rows * units; i += kQThreads) {
+        const unsigned rr = i / units, u = i - rr * units, h = u / upr, c = u - h * upr;
+        const int64_t r = row0 + rr;
+        const int64_t base = (r * n_heads + h) * head_dim;
+        const int pos = positions[r];
+        const bool in_table = pos >= 0 && pos < n_positions;
+        if (!in_table) atomicOr(err, HS_DEVERR_ROPE_RANGE);  // recorded; the row is copied unrotated
+        if (c >= rot) {
+            const int64_t at = base + rotary_dim + (c - rot) * 8u;
+            *reinterpret_cast<uint4 *>(out + at) = *reinterpret_cast<const uint4 *>(x + at);
+            continue;
+        }
+        const uint4 w1 = *reinterpret_cast<const uint4 *>(x + base + c * 8u), w2 = *reinterpret_cast<const uint4 *>(x + base + half + c * 8u);
+        uint32_t o1[4] = {w1.x, w1.y, w1.z, w1.w}, o2[4] = {w2.x, w2.y, w2.z, w2.w};
+        if (in_table) {
+            uint32_t sw[4], cw[4];
+            load_sincos8(sin + static_cast<int64_t>(pos) * half + c * 8u, cos + static_cast<int64_t>(pos) * half + c * 8u, sw, cw);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t a = o1[k], b = o2[k];
+                o1[k] = rope_pair(a, b, sw[k], cw[k], true);
+                o2[k] = rope_pair(b, a, sw[k], cw[k], false);
+            }
+        }
+        *reinterpret_cast<uint4 *>(out + base + c * 8u) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+        *reinterpret_cast<uint4 *>(out + base + half + c * 8u) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+    }
 }
 
 // Optional per-head RMS norm of K fused into quantise-on-write (weight == NULL: off).
@@ -107,6 +200,13 @@ struct KNormArgs {
     uint16_t *k_out;      // optional bf16 [n_seqs, n_tokens, n_kv_heads, head_dim]: the normed, rotated keys
     int pos_bias;         // added to dst_pos[s]: -1 when the caller hands the attended lengths instead of positions
 };
+
+// 8 norm weights, `add` (0 or 1) added to each
+__device__ __forceinline__ void load_weight8(const float *w, float add, float (&out)[8]) {
+    const float4 a = *reinterpret_cast<const float4 *>(w), b = *reinterpret_cast<const float4 *>(w + 4);
+    out[0] = a.x + add; out[1] = a.y + add; out[2] = a.z + add; out[3] = a.w + add;
+    out[4] = b.x + add; out[5] = b.y + add; out[6] = b.z + add; out[7] = b.w + add;
+}
 
 // ---- quantise-on-write into a cache view ----------------------------------------------------------------
 // E = elements per thread: 16 for long writes (prefill: bound by instruction issue, so the per-chunk costs are paid
@@ -120,8 +220,8 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
     // a decode launch that follows as a programmatic dependent may start now (it waits for this grid's completion before
     // it reads the cache); a no-op for every other successor
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ float smid[256];
-    fill_midpoints(KIND, smid);
+    __shared__ IndexTable<KIND> tab;
+    tab.fill();
     __syncthreads();
     // grid: x = groups of kUnroll * 256 E-element chunks of one sequence's new rows, y = 2 * sequence + (0: K, 1: V).
     // A thread owns E consecutive elements of a (token, head) row (16-byte loads; at E = 16 one 16-byte store of int8
@@ -140,8 +240,8 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
     const int tpb = view.block / E;
     const int bpr = D / view.block;  // blocks per (token, head) row
     const int cpr_shift = __ffs(static_cast<int>(cpr)) - 1, block_shift = __ffs(view.block) - 1;
-    const bool h_pow2 = (H & (H - 1)) == 0;
-    const int h_shift = __ffs(H) - 1;
+    const bool h_pow2 = (H & (H - 1)) == 0, page_pow2 = (view.page_tokens & (view.page_tokens - 1)) == 0;
+    const int h_shift = __ffs(H) - 1, page_shift = __ffs(view.page_tokens) - 1;
 #pragma unroll 2
     for (int u = 0; u < kUnroll; ++u) {
         const uint32_t chunk = (blockIdx.x * static_cast<uint32_t>(kUnroll) + u) * static_cast<uint32_t>(kQThreads) + threadIdx.x;
@@ -154,7 +254,7 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
         const int h = static_cast<int>(row_in_seq - static_cast<uint32_t>(t) * static_cast<uint32_t>(H));
         const int64_t row = static_cast<int64_t>(s) * n_tokens * H + row_in_seq;  // (seq, token, head)
         const int pos = base_pos + t;
-        const int page = pos / view.page_tokens;
+        const int page = page_pow2 ? pos >> page_shift : pos / view.page_tokens;
         bool ok = live && pos >= 0 && page < view.pages_per_seq;
         if (!is_v && sin != nullptr && (pos < 0 || pos >= n_positions)) ok = false;
         if (live && !ok) atomicOr(err, HS_DEVERR_KV_WRITE_RANGE);  // recorded, access skipped
@@ -187,29 +287,23 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
                 const int dd = d0 + 8 * part;
                 // the normed chunk as bf16 pairs (one packed conversion per pair = the one rounding to the model dtype), rotated in
                 // packed bf16 arithmetic like load_row8_rope: the same values as the scalar form, bit for bit
+                float wt[8];
+                load_weight8(kn.weight + dd, add, wt);
                 uint32_t ow[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    ow[i] = pack_bf16(x[8 * part + 2 * i] * rrms * (kn.weight[dd + 2 * i] + add), x[8 * part + 2 * i + 1] * rrms * (kn.weight[dd + 2 * i + 1] + add));
+                for (int i = 0; i < 4; ++i) ow[i] = pack_bf16(x[8 * part + 2 * i] * rrms * wt[2 * i], x[8 * part + 2 * i + 1] * rrms * wt[2 * i + 1]);
                 if (rope && dd < rotary_dim) {
                     const bool first = dd < half;
                     const int pd = first ? dd + half : dd - half;  // the rotation partner's chunk, normed the same way
                     float p8[8];
                     unpack8_bf16(*reinterpret_cast<const uint4 *>(src + pd), p8);
+                    load_weight8(kn.weight + pd, add, wt);
                     const int j0 = first ? dd : dd - half;
-                    const uint16_t *srow = sin + static_cast<int64_t>(pos) * half + j0;
-                    const uint16_t *crow = cos + static_cast<int64_t>(pos) * half + j0;
+                    uint32_t sw[4], cw[4];
+                    load_sincos8(sin + static_cast<int64_t>(pos) * half + j0, cos + static_cast<int64_t>(pos) * half + j0, sw, cw);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const uint32_t pw = pack_bf16(p8[2 * i] * rrms * (kn.weight[pd + 2 * i] + add), p8[2 * i + 1] * rrms * (kn.weight[pd + 2 * i + 1] + add));
-                        const uint32_t sw = static_cast<uint32_t>(srow[2 * i]) | (static_cast<uint32_t>(srow[2 * i + 1]) << 16);
-                        const uint32_t cw = static_cast<uint32_t>(crow[2 * i]) | (static_cast<uint32_t>(crow[2 * i + 1]) << 16);
-                        const __nv_bfloat162 own = *reinterpret_cast<const __nv_bfloat162 *>(&ow[i]), par = *reinterpret_cast<const __nv_bfloat162 *>(&pw);
-                        const __nv_bfloat162 s2 = *reinterpret_cast<const __nv_bfloat162 *>(&sw), c2 = *reinterpret_cast<const __nv_bfloat162 *>(&cw);
-                        const __nv_bfloat162 oc = __hmul2(own, c2), ps = __hmul2(par, s2);
-                        const __nv_bfloat162 r = first ? __hsub2(oc, ps) : __hadd2(ps, oc);  // x1*cos - x2*sin | x1*sin + x2*cos
-                        ow[i] = *reinterpret_cast<const uint32_t *>(&r);
-                    }
+                    for (int i = 0; i < 4; ++i)
+                        ow[i] = rope_pair(ow[i], pack_bf16(p8[2 * i] * rrms * wt[2 * i], p8[2 * i + 1] * rrms * wt[2 * i + 1]), sw[i], cw[i], first);
                 }
                 if (kn.k_out != nullptr && ok)  // the normed, rotated keys in bf16, for a prompt's own attention
                     *reinterpret_cast<uint4 *>(kn.k_out + row * D + dd) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
@@ -241,8 +335,8 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
             continue;
         }
         constexpr int QK = KIND == HS_KV_BF16 ? HS_KV_INT8 : KIND;
-        int c[E];
-        float a = quantize_n<QK, E>(x, tpb, view.scale_dtype, smid, c);
+        CodeWords<QK, E> c;
+        float a = quantize_n<QK, E>(x, tpb, view.scale_dtype, tab, c);
         if (!ok) continue;
         uint8_t *codes = reinterpret_cast<uint8_t *>(data_pages[pidx]);
         void *scales = scale_pages[pidx];
@@ -250,76 +344,81 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
         const int64_t e0 = in_page * D + d0;
         if constexpr (E == 8) {
             store_codes8<QK>(codes, e0, e0 + 8, c, true);
+        } else if constexpr (QK == HS_KV_INT8) {
+            *reinterpret_cast<uint4 *>(codes + e0) = make_uint4(c.w[0], c.w[1], c.w[2], c.w[3]);
         } else {
-#pragma unroll
-            for (int part = 0; part < E / 16; ++part) {
-                const int *cp = c + 16 * part;
-                if (QK == HS_KV_INT8) {
-                    uint4 w;
-                    w.x = cp[0] | (cp[1] << 8) | (cp[2] << 16) | (cp[3] << 24);
-                    w.y = cp[4] | (cp[5] << 8) | (cp[6] << 16) | (cp[7] << 24);
-                    w.z = cp[8] | (cp[9] << 8) | (cp[10] << 16) | (cp[11] << 24);
-                    w.w = cp[12] | (cp[13] << 8) | (cp[14] << 16) | (cp[15] << 24);
-                    reinterpret_cast<uint4 *>(codes + e0)[part] = w;
-                } else {  // the even element in the high nibble
-                    uint2 w;
-                    w.x = ((cp[0] << 4) | cp[1]) | (((cp[2] << 4) | cp[3]) << 8) | (((cp[4] << 4) | cp[5]) << 16) | (((cp[6] << 4) | cp[7]) << 24);
-                    w.y = ((cp[8] << 4) | cp[9]) | (((cp[10] << 4) | cp[11]) << 8) | (((cp[12] << 4) | cp[13]) << 16) | (((cp[14] << 4) | cp[15]) << 24);
-                    reinterpret_cast<uint2 *>(codes + (e0 >> 1))[part] = w;
-                }
-            }
+            *reinterpret_cast<uint2 *>(codes + (e0 >> 1)) = make_uint2(c.w[0], c.w[1]);
         }
     }
 }
 
 // ---- gather-dequantise (LayerKVCache::get compatibility read) ------------------------------------------------
-__global__ void __launch_bounds__(kQThreads) kv_gather_kernel(ViewDev view, const int32_t *__restrict__ seq_lens, int n_seqs,
-                                                              int out_tokens, uint16_t *__restrict__ k_out,
-                                                              uint16_t *__restrict__ v_out) {
-    __shared__ float stab[16];
-    if (view.kind >= HS_KV_NF4 && threadIdx.x < 16) stab[threadIdx.x] = view.kind == HS_KV_NF4 ? c_nf4[threadIdx.x] : c_fp4[threadIdx.x];
+// grid: x = groups of kGatherChunks * 256 chunks of 8 elements of one sequence's rows, y = 2 * sequence + (0: K, 1: V).  A thread
+// has kGatherChunks loads in flight; shifts and 32-bit arithmetic in place of the 64-bit divisions per 8 elements it had.
+constexpr int kGatherChunks = 4;
+template <int KIND>
+__global__ void __launch_bounds__(kQThreads) kv_gather_kernel(ViewDev view, const int32_t *__restrict__ seq_lens, int out_tokens,
+                                                              uint16_t *__restrict__ k_out, uint16_t *__restrict__ v_out) {
+    __shared__ ValueTable<KIND> tab;
+    tab.fill();
     __syncthreads();
-    const bool is_v = blockIdx.y == 1;
+    const bool is_v = (blockIdx.y & 1u) != 0;
+    const int s = static_cast<int>(blockIdx.y >> 1);
     const int D = view.head_dim, H = view.n_kv_heads;
-    const int cpr = D / 8;
-    const int64_t chunk = static_cast<int64_t>(blockIdx.x) * kQThreads + threadIdx.x;
-    const int64_t total = static_cast<int64_t>(n_seqs) * out_tokens * H * cpr;
-    if (chunk >= total) return;
-    const int d0 = static_cast<int>(chunk % cpr) * 8;
-    const int64_t row = chunk / cpr;
-    const int h = static_cast<int>(row % H);
-    const int64_t st = row / H;
-    const int t = static_cast<int>(st % out_tokens);
-    const int s = static_cast<int>(st / out_tokens);
-    uint4 w = make_uint4(0, 0, 0, 0);
-    const int page = t / view.page_tokens;
-    if (t < seq_lens[s] && page < view.pages_per_seq) {
-        const int64_t pidx = static_cast<int64_t>(s) * view.pages_per_seq + page;
+    const int cpr_shift = __ffs(D) - 4;   // head_dim is a power of two: 8-element chunks per (token, head) row
+    const int block_shift = __ffs(view.block) - 1, bpr = D / view.block;
+    const bool page_pow2 = (view.page_tokens & (view.page_tokens - 1)) == 0, h_pow2 = (H & (H - 1)) == 0;
+    const int page_shift = __ffs(view.page_tokens) - 1, h_shift = __ffs(H) - 1;
+    const int64_t total = (static_cast<int64_t>(out_tokens) * H) << cpr_shift;
+    const int64_t chunk0 = static_cast<int64_t>(blockIdx.x) * (kGatherChunks * kQThreads) + threadIdx.x;
+    const int len = min(seq_lens[s], out_tokens);
+    void *const *data_pages = (is_v ? view.v_pages : view.k_pages) + static_cast<int64_t>(s) * view.pages_per_seq;
+    void *const *scale_pages = KIND == HS_KV_BF16 ? nullptr : (is_v ? view.v_scale_pages : view.k_scale_pages) + static_cast<int64_t>(s) * view.pages_per_seq;
+    uint4 w[kGatherChunks];
+    float a[kGatherChunks];
+    bool live[kGatherChunks];
+#pragma unroll
+    for (int u = 0; u < kGatherChunks; ++u) {
+        const int64_t chunk = chunk0 + u * kQThreads;
+        w[u] = make_uint4(0, 0, 0, 0);
+        a[u] = 0.0f;
+        live[u] = false;
+        if (chunk >= total) continue;
+        const int d0 = static_cast<int>(chunk & ((1 << cpr_shift) - 1)) * 8;
+        const int64_t row = chunk >> cpr_shift;
+        const int t = static_cast<int>(h_pow2 ? row >> h_shift : row / H);
+        const int h = static_cast<int>(row - static_cast<int64_t>(t) * H);
+        const int page = page_pow2 ? t >> page_shift : t / view.page_tokens;
+        live[u] = t < len && page < view.pages_per_seq;
+        if (!live[u]) continue;
         const int64_t in_page = static_cast<int64_t>(t - page * view.page_tokens) * H + h;
-        const void *data = (is_v ? view.v_pages : view.k_pages)[pidx];
-        if (view.kind == HS_KV_BF16) {
-            w = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(data) + in_page * D + d0);
+        const unsigned char *data = reinterpret_cast<const unsigned char *>(data_pages[page]);
+        if constexpr (KIND == HS_KV_BF16) {
+            w[u] = *reinterpret_cast<const uint4 *>(data + (in_page * D + d0) * 2);
         } else {
-            const void *scales = (is_v ? view.v_scale_pages : view.k_scale_pages)[pidx];
-            const float a = load_scale(scales, in_page * (D / view.block) + d0 / view.block, view.scale_dtype);
-            float v[8];
-            const uint8_t *codes = reinterpret_cast<const uint8_t *>(data);
-            if (view.kind == HS_KV_INT8) {
-                uint2 cw = *reinterpret_cast<const uint2 *>(codes + in_page * D + d0);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(code8(((i < 4 ? cw.x : cw.y) >> (8 * (i & 3))) & 0xff), a);
+            a[u] = load_scale(scale_pages[page], in_page * bpr + (d0 >> block_shift), view.scale_dtype);
+            if constexpr (KIND == HS_KV_INT8) {
+                const uint2 c = *reinterpret_cast<const uint2 *>(data + in_page * D + d0);
+                w[u].x = c.x; w[u].y = c.y;
             } else {
-                uint32_t cw = *reinterpret_cast<const uint32_t *>(codes + ((in_page * D + d0) >> 1));
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    int byte = (cw >> (8 * (i >> 1))) & 0xff;
-                    v[i] = __fmul_rn(stab[(i & 1) ? (byte & 0xf) : (byte >> 4)], a);
-                }
+                w[u].x = *reinterpret_cast<const uint32_t *>(data + ((in_page * D + d0) >> 1));
             }
-            w.x = pack_bf16(v[0], v[1]); w.y = pack_bf16(v[2], v[3]); w.z = pack_bf16(v[4], v[5]); w.w = pack_bf16(v[6], v[7]);
         }
     }
-    *reinterpret_cast<uint4 *>((is_v ? v_out : k_out) + row * D + d0) = w;
+#pragma unroll
+    for (int u = 0; u < kGatherChunks; ++u) {
+        const int64_t chunk = chunk0 + u * kQThreads;
+        if (chunk >= total) return;
+        if constexpr (KIND != HS_KV_BF16) {
+            float v[8];
+            tab.values8(make_uint2(w[u].x, w[u].y), v);
+            uint32_t o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = live[u] ? pack_bf16(__fmul_rn(v[2 * i], a[u]), __fmul_rn(v[2 * i + 1], a[u])) : 0u;
+            w[u] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        *reinterpret_cast<uint4 *>((is_v ? v_out : k_out) + ((static_cast<int64_t>(s) * total + chunk) << 3)) = w[u];
+    }
 }
 
 }  // namespace hs
@@ -344,12 +443,17 @@ int32_t hs_quantize_blockwise(int32_t kind, const void *src, int32_t dtype, int6
     if (!aligned(codes, kind == HS_KV_INT8 ? 8 : 4)) return fail(HS_ERR_ARG, "hs_quantize_blockwise: codes must be 8-byte aligned");
     const int vec_ok = aligned(src, 16) ? 1 : 0;
     const int64_t chunks = (n + 7) / 8;
-    // whole quantisation blocks per CTA: kQThreads*8 elements is a multiple of every supported block
-    const unsigned grid = static_cast<unsigned>((chunks + kQThreads - 1) / kQThreads);
+    // whole quantisation blocks per warp: 32 * 8 elements are a multiple of every supported block
+    const unsigned grid = static_cast<unsigned>((chunks + kQThreads * kFlatChunks - 1) / (kQThreads * kFlatChunks));
     cudaStream_t s = as_stream(stream);
-    if (kind == HS_KV_INT8) quantize_flat_kernel<HS_KV_INT8><<<grid, kQThreads, 0, s>>>(src, dtype, n, block, scale_dtype, codes, absmax, vec_ok);
-    else if (kind == HS_KV_NF4) quantize_flat_kernel<HS_KV_NF4><<<grid, kQThreads, 0, s>>>(src, dtype, n, block, scale_dtype, codes, absmax, vec_ok);
-    else quantize_flat_kernel<HS_KV_FP4><<<grid, kQThreads, 0, s>>>(src, dtype, n, block, scale_dtype, codes, absmax, vec_ok);
+#define HS_QUANT(K, T) quantize_flat_kernel<K, T><<<grid, kQThreads, 0, s>>>(src, n, block, scale_dtype, codes, absmax, vec_ok)
+#define HS_QUANT_T(K) do { if (dtype == HS_DTYPE_BF16) HS_QUANT(K, HS_DTYPE_BF16); else if (dtype == HS_DTYPE_F16) HS_QUANT(K, HS_DTYPE_F16); \
+                           else HS_QUANT(K, HS_DTYPE_F32); } while (0)
+    if (kind == HS_KV_INT8) HS_QUANT_T(HS_KV_INT8);
+    else if (kind == HS_KV_NF4) HS_QUANT_T(HS_KV_NF4);
+    else HS_QUANT_T(HS_KV_FP4);
+#undef HS_QUANT_T
+#undef HS_QUANT
     return check_launch("hs_quantize_blockwise");
 }
 
@@ -367,8 +471,17 @@ int32_t hs_dequantize_blockwise(int32_t kind, const uint8_t *codes, const void *
     if (!aligned(out, dtype == HS_DTYPE_F32 ? 4 : 2) || !aligned(absmax, scale_dtype == HS_SCALE_F16 ? 2 : 4))
         return fail(HS_ERR_ARG, "hs_dequantize_blockwise: misaligned pointer");
     const int64_t chunks = (n + 7) / 8;
-    const unsigned grid = static_cast<unsigned>((chunks + kQThreads - 1) / kQThreads);
-    dequantize_flat_kernel<<<grid, kQThreads, 0, as_stream(stream)>>>(kind, codes, absmax, n, block, scale_dtype, out, dtype);
+    const unsigned grid = static_cast<unsigned>((chunks + kQThreads * kFlatChunks - 1) / (kQThreads * kFlatChunks));
+    const int vec_ok = aligned(codes, kind == HS_KV_INT8 ? 8 : 4) && aligned(out, 16) ? 1 : 0;
+    cudaStream_t s = as_stream(stream);
+#define HS_DEQUANT(K, T) dequantize_flat_kernel<K, T><<<grid, kQThreads, 0, s>>>(codes, absmax, n, block, scale_dtype, out, vec_ok)
+#define HS_DEQUANT_T(K) do { if (dtype == HS_DTYPE_BF16) HS_DEQUANT(K, HS_DTYPE_BF16); else if (dtype == HS_DTYPE_F16) HS_DEQUANT(K, HS_DTYPE_F16); \
+                             else HS_DEQUANT(K, HS_DTYPE_F32); } while (0)
+    if (kind == HS_KV_INT8) HS_DEQUANT_T(HS_KV_INT8);
+    else if (kind == HS_KV_NF4) HS_DEQUANT_T(HS_KV_NF4);
+    else HS_DEQUANT_T(HS_KV_FP4);
+#undef HS_DEQUANT_T
+#undef HS_DEQUANT
     return check_launch("hs_dequantize_blockwise");
 }
 
@@ -385,11 +498,14 @@ int32_t hs_rope_apply(const void *x, void *out, const void *sin, const void *cos
     if (x == out && rotary_dim > 0) return fail(HS_ERR_ARG, "hs_rope_apply: in-place rotation is not supported (a lane reads its partner half)");
     int *err = device_error_word();
     if (!err) return fail(HS_ERR_DEVICE, "hs_rope_apply: device error word unavailable");
-    const int64_t chunks = n_rows * n_heads * (head_dim / 8);
-    const unsigned grid = static_cast<unsigned>((chunks + kQThreads - 1) / kQThreads);
+    const int units = (rotary_dim / 16 + (head_dim - rotary_dim) / 8) * n_heads;  // work units of a row
+    // about four units per thread; never more than the grid can be addressed with
+    int64_t rows_per_block = max(1, min(1 << 16, 4 * kQThreads / max(1, units)));
+    if ((n_rows + rows_per_block - 1) / rows_per_block < 2 * sm_count()) rows_per_block = max(1, kQThreads / max(1, units));  // few rows: spread them
+    const unsigned grid = static_cast<unsigned>((n_rows + rows_per_block - 1) / rows_per_block);
     rope_kernel<<<grid, kQThreads, 0, as_stream(stream)>>>(
         reinterpret_cast<const uint16_t *>(x), reinterpret_cast<uint16_t *>(out), reinterpret_cast<const uint16_t *>(sin),
-        reinterpret_cast<const uint16_t *>(cos), positions, n_rows, n_heads, head_dim, rotary_dim, n_positions, err);
+        reinterpret_cast<const uint16_t *>(cos), positions, n_rows, n_heads, head_dim, rotary_dim, n_positions, static_cast<int>(rows_per_block), err);
     return check_launch("hs_rope_apply");
 }
 
@@ -419,7 +535,7 @@ static int32_t kv_write_impl(const char *who, const hs_kv_view *view, const void
     if (!err) return fail(HS_ERR_DEVICE, "%s: device error word unavailable", who);
     const uint16_t *k = reinterpret_cast<const uint16_t *>(k_new), *v = reinterpret_cast<const uint16_t *>(v_new);
     const uint16_t *sn = reinterpret_cast<const uint16_t *>(sin), *cs = reinterpret_cast<const uint16_t *>(cos);
-#define HS_KV_WRITE(K) do { if (wide) kv_write_kernel<K, HS_KV_WRITE_WIDE><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); \
+#define HS_KV_WRITE(K) do { if (wide) kv_write_kernel<K, 16><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); \
                             else kv_write_kernel<K, 8><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); } while (0)
     switch (view->kind) {
         case HS_KV_BF16: HS_KV_WRITE(HS_KV_BF16); break;
@@ -467,10 +583,28 @@ int32_t hs_kv_gather_dequantize(const hs_kv_view *view, const int32_t *seq_lens,
     if (!seq_lens || !k_out || !v_out) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: NULL pointer");
     if (!aligned(k_out, 16) || !aligned(v_out, 16)) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: outputs must be 16-byte aligned");
     ViewDev d = to_dev(view);
-    const int64_t chunks = static_cast<int64_t>(n_seqs) * out_tokens * d.n_kv_heads * (d.head_dim / 8);
-    dim3 grid(static_cast<unsigned>((chunks + kQThreads - 1) / kQThreads), 2);
-    kv_gather_kernel<<<grid, kQThreads, 0, as_stream(stream)>>>(d, seq_lens, n_seqs, out_tokens,
-                                                               reinterpret_cast<uint16_t *>(k_out), reinterpret_cast<uint16_t *>(v_out));
+    if (n_seqs > 32767) {  // the grid's second dimension holds 2 * 32767 rows: the rest in calls of their own
+        const int64_t step = static_cast<int64_t>(32767) * out_tokens * d.n_kv_heads * d.head_dim * 2;
+        hs_kv_view rest = *view;
+        const int64_t pages = static_cast<int64_t>(32767) * view->pages_per_seq;
+        rest.k_pages += pages;
+        rest.v_pages += pages;
+        if (rest.k_scale_pages) rest.k_scale_pages += pages;
+        if (rest.v_scale_pages) rest.v_scale_pages += pages;
+        if (int32_t st = hs_kv_gather_dequantize(view, seq_lens, 32767, out_tokens, k_out, v_out, stream)) return st;
+        return hs_kv_gather_dequantize(&rest, seq_lens + 32767, n_seqs - 32767, out_tokens, static_cast<char *>(k_out) + step,
+                                       static_cast<char *>(v_out) + step, stream);
+    }
+    const int64_t chunks = static_cast<int64_t>(out_tokens) * d.n_kv_heads * (d.head_dim / 8);
+    dim3 grid(static_cast<unsigned>((chunks + kGatherChunks * kQThreads - 1) / (kGatherChunks * kQThreads)), 2u * static_cast<unsigned>(n_seqs));
+    cudaStream_t s = as_stream(stream);
+    uint16_t *ko = reinterpret_cast<uint16_t *>(k_out), *vo = reinterpret_cast<uint16_t *>(v_out);
+    switch (view->kind) {
+        case HS_KV_BF16: kv_gather_kernel<HS_KV_BF16><<<grid, kQThreads, 0, s>>>(d, seq_lens, out_tokens, ko, vo); break;
+        case HS_KV_INT8: kv_gather_kernel<HS_KV_INT8><<<grid, kQThreads, 0, s>>>(d, seq_lens, out_tokens, ko, vo); break;
+        case HS_KV_NF4: kv_gather_kernel<HS_KV_NF4><<<grid, kQThreads, 0, s>>>(d, seq_lens, out_tokens, ko, vo); break;
+        default: kv_gather_kernel<HS_KV_FP4><<<grid, kQThreads, 0, s>>>(d, seq_lens, out_tokens, ko, vo); break;
+    }
     return check_launch("hs_kv_gather_dequantize");
 }
 
