@@ -211,7 +211,12 @@ __device__ __forceinline__ void load_weight8(const float *w, float add, float (&
 // ---- quantise-on-write into a cache view ----------------------------------------------------------------
 // E = elements per thread: 16 for long writes (prefill: bound by instruction issue, so the per-chunk costs are paid
 // half as often), 8 for short ones (a decode step's single token per sequence: latency matters, not throughput).
-template <int KIND, int E>
+//
+// Issue bound, not HBM bound, as first written (523 warp instructions per 16-element chunk, a fifth of the stalls for
+// instruction fetch).  Where a block's rows lie in one page and need no rotation or norm (V always; K that arrives finished) the
+// source and the cache have the same layout: one linear copy-and-quantise with all of a thread's loads in flight and no
+// (token, head) split; the norm is an instantiation of its own.
+template <int KIND, int E, bool NORM>
 __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const uint16_t *__restrict__ k_new,
                                                              const uint16_t *__restrict__ v_new, int n_seqs, int n_tokens,
                                                              const int32_t *__restrict__ dst_pos,
@@ -242,7 +247,56 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
     const int cpr_shift = __ffs(static_cast<int>(cpr)) - 1, block_shift = __ffs(view.block) - 1;
     const bool h_pow2 = (H & (H - 1)) == 0, page_pow2 = (view.page_tokens & (view.page_tokens - 1)) == 0;
     const int h_shift = __ffs(H) - 1, page_shift = __ffs(view.page_tokens) - 1;
-#pragma unroll 2
+    if constexpr (E == 16) {
+        const uint32_t c0 = blockIdx.x * static_cast<uint32_t>(kUnroll * kQThreads), c1 = min(c0 + static_cast<uint32_t>(kUnroll * kQThreads), total);
+        const uint32_t hc = static_cast<uint32_t>(H) * cpr;                 // chunks per token
+        const int pos0 = base_pos + static_cast<int>(c0 / hc), pos1 = base_pos + static_cast<int>((c1 - 1u) / hc);
+        const int page = pos0 / view.page_tokens;
+        if (c0 >= total) return;
+        if ((is_v || (!NORM && sin == nullptr)) && base_pos >= 0 && pos1 / view.page_tokens == page && page < view.pages_per_seq) {
+            const int64_t pidx = static_cast<int64_t>(s) * view.pages_per_seq + page;
+            // element offset between the source rows of this sequence and their place in the page
+            const int64_t shift = (static_cast<int64_t>(base_pos) - static_cast<int64_t>(page) * view.page_tokens) * H * D;
+            const uint4 *src = reinterpret_cast<const uint4 *>((is_v ? v_new : k_new) + static_cast<int64_t>(s) * n_tokens * H * D);
+            uint4 w[kUnroll][2];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const uint32_t chunk = c0 + u * kQThreads + threadIdx.x;
+                w[u][0] = w[u][1] = make_uint4(0, 0, 0, 0);
+                if (chunk < total) {
+                    w[u][0] = src[2 * static_cast<int64_t>(chunk)];
+                    w[u][1] = src[2 * static_cast<int64_t>(chunk) + 1];
+                }
+            }
+            uint8_t *data = reinterpret_cast<uint8_t *>(data_pages[pidx]);
+            void *scales = KIND == HS_KV_BF16 ? nullptr : scale_pages[pidx];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const uint32_t chunk = c0 + u * kQThreads + threadIdx.x;
+                const int64_t e0 = shift + static_cast<int64_t>(chunk) * 16;
+                if constexpr (KIND == HS_KV_BF16) {
+                    if (chunk < total) {
+                        reinterpret_cast<uint4 *>(data + 2 * e0)[0] = w[u][0];
+                        reinterpret_cast<uint4 *>(data + 2 * e0)[1] = w[u][1];
+                    }
+                } else {
+                    float amax = fmaxf(absmax8_bf16(w[u][0]), absmax8_bf16(w[u][1]));
+                    for (int o = 1; o < tpb; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                    if (chunk >= total) continue;
+                    float x[16];
+                    unpack8_bf16(w[u][0], *reinterpret_cast<float(*)[8]>(&x[0]));
+                    unpack8_bf16(w[u][1], *reinterpret_cast<float(*)[8]>(&x[8]));
+                    CodeWords<KIND, 16> c;
+                    const float a = quantize_given_max<KIND, 16>(x, amax, view.scale_dtype, tab, c);
+                    if ((threadIdx.x & (tpb - 1)) == 0) store_scale(scales, e0 >> block_shift, view.scale_dtype, a);
+                    if constexpr (KIND == HS_KV_INT8) *reinterpret_cast<uint4 *>(data + e0) = make_uint4(c.w[0], c.w[1], c.w[2], c.w[3]);
+                    else *reinterpret_cast<uint2 *>(data + (e0 >> 1)) = make_uint2(c.w[0], c.w[1]);
+                }
+            }
+            return;
+        }
+    }
+#pragma unroll 1
     for (int u = 0; u < kUnroll; ++u) {
         const uint32_t chunk = (blockIdx.x * static_cast<uint32_t>(kUnroll) + u) * static_cast<uint32_t>(kQThreads) + threadIdx.x;
         if (chunk - threadIdx.x >= total) break;  // (uniform over the block)
@@ -260,7 +314,7 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
         if (live && !ok) atomicOr(err, HS_DEVERR_KV_WRITE_RANGE);  // recorded, access skipped
         const uint16_t *src = (is_v ? v_new : k_new) + row * D;
         float x[E];
-        if (kn.weight != nullptr && !is_v) {
+        if (NORM && !is_v) {
             // ---- K with its per-head RMS norm fused in (qwen3_5.rs:1077-1091; llama.rs:929-992): the row's sum of squares is
             // formed exactly as hs_qk_norm_rope forms it (an 8-element chain per 16-byte chunk, then pairwise over the chunks
             // of the row), so the normed, rotated values - and with them the stored codes - equal the two-kernel route bit
@@ -535,8 +589,9 @@ static int32_t kv_write_impl(const char *who, const hs_kv_view *view, const void
     if (!err) return fail(HS_ERR_DEVICE, "%s: device error word unavailable", who);
     const uint16_t *k = reinterpret_cast<const uint16_t *>(k_new), *v = reinterpret_cast<const uint16_t *>(v_new);
     const uint16_t *sn = reinterpret_cast<const uint16_t *>(sin), *cs = reinterpret_cast<const uint16_t *>(cos);
-#define HS_KV_WRITE(K) do { if (wide) kv_write_kernel<K, 16><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); \
-                            else kv_write_kernel<K, 8><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); } while (0)
+#define HS_KV_WRITE_N(K, N) do { if (wide) kv_write_kernel<K, 16, N><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); \
+                                 else kv_write_kernel<K, 8, N><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); } while (0)
+#define HS_KV_WRITE(K) do { if (kn.weight != nullptr) HS_KV_WRITE_N(K, true); else HS_KV_WRITE_N(K, false); } while (0)
     switch (view->kind) {
         case HS_KV_BF16: HS_KV_WRITE(HS_KV_BF16); break;
         case HS_KV_INT8: HS_KV_WRITE(HS_KV_INT8); break;
@@ -544,6 +599,7 @@ static int32_t kv_write_impl(const char *who, const hs_kv_view *view, const void
         default: HS_KV_WRITE(HS_KV_FP4); break;
     }
 #undef HS_KV_WRITE
+#undef HS_KV_WRITE_N
     return check_launch(who);
 }
 

@@ -177,20 +177,23 @@ struct CodeWords {
     }
 };
 
-// Quantise the N values of this thread; `tpb` consecutive lanes (a power of two <= 32) share a block.
+// ---- quantise the N values of a thread; `tpb` consecutive lanes (a power of two <= 32) share a block ----
 // Returns the stored scale (already rounded in f16 mode); `cw` receives N indices.
 //
-// u8 codes, two values per instruction: y = x / absmax, t = 127 y, and t + (1.5 * 2^23 + 127) holds the candidate code in its
-// low byte (a NaN's low byte is 255, the index the scalar form gives it).  Only where a candidate's t lies within 1e-4 of a
-// half-integer (the roundings are off by less than 2e-5) are the true midpoints consulted, value by value; so is a block
-// whose values leave [-1, 1].  Issue bound: 43 -> about 20 instructions per element of the write kernel together with it.
+// u8 codes, two values per instruction: t = x (127 / absmax), and t + (1.5 * 2^23 + 127) holds the candidate code in its low byte
+// (a NaN's low byte is 255, the index the scalar form gives it).  Only where a candidate's t lies within 1e-4 of a half-integer
+// (the roundings are off by less than 4e-5) are the true midpoints consulted, value by value; so is a block whose values leave
+// [-1, 1].  That path is a call: inlined 16 times it made the write kernel miss the instruction cache.
+template <typename Index>
+__device__ __noinline__ uint32_t index_int8_word(float x0, float x1, float x2, float x3, float inv, const Index &index) {
+    return static_cast<uint32_t>(index(__fmul_rn(x0, inv))) | static_cast<uint32_t>(index(__fmul_rn(x1, inv))) << 8 |
+           static_cast<uint32_t>(index(__fmul_rn(x2, inv))) << 16 | static_cast<uint32_t>(index(__fmul_rn(x3, inv))) << 24;
+}
+
+// The codes of the N values of this thread, given the largest magnitude of their block (over all its lanes).
 template <int KIND, int N, typename Index>
-__device__ __forceinline__ float quantize_n(const float (&x)[N], int tpb, int scale_dtype, const Index &index, CodeWords<KIND, N> &cw) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < N; ++i) amax = fmaxf(amax, fabsf(x[i]));
-    for (int o = 1; o < tpb; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    float a = scale_dtype == HS_SCALE_F16 ? f16_sat_round(amax) : amax;
+__device__ __forceinline__ float quantize_given_max(const float (&x)[N], float amax, int scale_dtype, const Index &index, CodeWords<KIND, N> &cw) {
+    const float a = scale_dtype == HS_SCALE_F16 ? f16_sat_round(amax) : amax;
     if (a == 0.0f) {
         const uint32_t zw = KIND == HS_KV_INT8 ? 0x7f7f7f7fu : (KIND == HS_KV_NF4 ? 0x77777777u : 0u);
 #pragma unroll
@@ -199,33 +202,24 @@ __device__ __forceinline__ float quantize_n(const float (&x)[N], int tpb, int sc
     }
     const float inv = __fdiv_rn(1.0f, a);
     if constexpr (KIND == HS_KV_INT8) {
-        const uint64_t inv2 = f2_pack(inv, inv), c127 = f2_pack(127.0f, 127.0f), magic = f2_pack(12583039.0f, 12583039.0f),
-                       unmagic = f2_pack(-12583039.0f, -12583039.0f), minus1 = f2_pack(-1.0f, -1.0f);
-        // largest distance of a t from its candidate; a scale that f16 cut short, or whose reciprocal overflows, lets t leave the
-        // range in which the low byte is the code
-        float off = __fmul_rn(amax, inv) > 1.002f ? 1.0f : 0.0f;
+        const float inv127 = __fmul_rn(inv, 127.0f);
+        const uint64_t scale = f2_pack(inv127, inv127), magic = f2_pack(12583039.0f, 12583039.0f), unmagic = f2_pack(-12583039.0f, -12583039.0f),
+                       minus1 = f2_pack(-1.0f, -1.0f);
+        // a scale that f16 cut short, or a reciprocal that overflows, lets t leave the range in which the low byte is the code
+        const float wide = __fmul_rn(amax, inv127) > 127.3f ? 1.0f : 0.0f;
 #pragma unroll
         for (int i = 0; i < N; i += 4) {
-            const uint64_t t0 = f2_mul(f2_mul(f2_pack(x[i], x[i + 1]), inv2), c127), t1 = f2_mul(f2_mul(f2_pack(x[i + 2], x[i + 3]), inv2), c127);
+            const uint64_t t0 = f2_mul(f2_pack(x[i], x[i + 1]), scale), t1 = f2_mul(f2_pack(x[i + 2], x[i + 3]), scale);
             const uint64_t m0 = f2_add(t0, magic), m1 = f2_add(t1, magic);
             float b[4], d[4];
             f2_unpack(m0, b[0], b[1]);
             f2_unpack(m1, b[2], b[3]);
             f2_unpack(f2_fma(f2_add(m0, unmagic), minus1, t0), d[0], d[1]);
             f2_unpack(f2_fma(f2_add(m1, unmagic), minus1, t1), d[2], d[3]);
-            off = fmaxf(fmaxf(off, fabsf(d[0])), fabsf(d[1]));
-            off = fmaxf(fmaxf(off, fabsf(d[2])), fabsf(d[3]));
             const uint32_t lo = __byte_perm(__float_as_uint(b[0]), __float_as_uint(b[1]), 0x0040), hi = __byte_perm(__float_as_uint(b[2]), __float_as_uint(b[3]), 0x0040);
             cw.w[i / 4] = __byte_perm(lo, hi, 0x5410);
-        }
-        if (off > 0.4999f) {
-#pragma unroll
-            for (int i = 0; i < N; i += 4) {
-                uint32_t w = 0;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) w |= static_cast<uint32_t>(index(__fmul_rn(x[i + e], inv))) << (8 * e);
-                cw.w[i / 4] = w;
-            }
+            const float off = fmaxf(fmaxf(fmaxf(wide, fabsf(d[0])), fabsf(d[1])), fmaxf(fabsf(d[2]), fabsf(d[3])));
+            if (off > 0.4999f) cw.w[i / 4] = index_int8_word(x[i], x[i + 1], x[i + 2], x[i + 3], inv, index);
         }
     } else {
 #pragma unroll
@@ -237,6 +231,21 @@ __device__ __forceinline__ float quantize_n(const float (&x)[N], int tpb, int sc
         }
     }
     return a;
+}
+template <int KIND, int N, typename Index>
+__device__ __forceinline__ float quantize_n(const float (&x)[N], int tpb, int scale_dtype, const Index &index, CodeWords<KIND, N> &cw) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) amax = fmaxf(amax, fabsf(x[i]));
+    for (int o = 1; o < tpb; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    return quantize_given_max<KIND, N>(x, amax, scale_dtype, index, cw);
+}
+// largest magnitude of 8 bf16 values (a NaN is passed over, as fmaxf passes over it)
+__device__ __forceinline__ float absmax8_bf16(const uint4 &w) {
+    const uint32_t ww[4] = {w.x & 0x7fff7fffu, w.y & 0x7fff7fffu, w.z & 0x7fff7fffu, w.w & 0x7fff7fffu};
+    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(ww);
+    const __nv_bfloat162 m = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
+    return fmaxf(fmaxf(__low2float(m), __high2float(m)), 0.0f);
 }
 
 __device__ __forceinline__ void store_scale(void *p, int64_t idx, int scale_dtype, float a) {
