@@ -1,4 +1,4 @@
-// Causal GQA prefill attention on the 5th-generation tensor cores (bf16; head_dim 128 first, head_dim 256 further down).
+// Causal GQA prefill attention on the 5th-generation tensor cores (bf16; head_dim 128 and 64 first, head_dim 256 further down).
 //
 // One CTA = two 128-row query tiles of one head (256 rows) sharing every K/V tile.  Roles (10 warps):
 //   warp 8  loader: TMA tensor loads (cp.async.bulk.tensor, 128-byte swizzle, no multicast) of the two Q tiles
@@ -30,13 +30,16 @@
 
 namespace hs {
 
-constexpr int kT5M = 128, kT5N = 128, kT5D = 128;
+constexpr int kT5M = 128, kT5N = 128;
 constexpr int kT5Stages = 2;
 constexpr int kT5BlockM = 2 * kT5M;  // two query tiles per CTA
 constexpr int kT5Threads = 320;
-constexpr int kT5TileBytes = kT5N * kT5D * 2;          // 32 KB: two 64-column halves of [128 rows][128 B]
-constexpr int kT5HalfBytes = kT5TileBytes / 2;
-constexpr int kT5SmemBytes = kT5TileBytes * (2 + 2 * kT5Stages) + 1024;  // two Q tiles, K/V ring, alignment slack
+constexpr int kT5HalfBytes = kT5N * 128;               // 16 KB: 64 columns of 128 rows, one swizzled box
+template <int D>
+struct T5Shape {                                       // head_dim 128: two boxes a tile; head_dim 64: one
+    static constexpr int kTileBytes = kT5N * D * 2;
+    static constexpr int kSmemBytes = kTileBytes * (2 + 2 * kT5Stages) + 1024;  // two Q tiles, K/V ring, alignment slack
+};
 constexpr long long kT5WaitCycles = 400000000LL;  // ~0.2 s: any legitimate wait is far below a millisecond
 constexpr float kT5RescaleThreshold = 8.0f;            // log2 units
 
@@ -173,17 +176,19 @@ __device__ __forceinline__ float t5_ex2(float x) {
 
 // Two 128-row query tiles (x = 0, 1) per CTA share every K/V tile.  Warps 0-3: softmax of tile 0, warps 4-7: softmax of
 // tile 1, warp 8: loader, warp 9: MMA issuer.  TMEM columns: S/P of tile x at 128x, O of tile x at 256 + 128x.
+template <int D>
 __global__ void __launch_bounds__(kT5Threads, 1)
 prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, uint16_t *__restrict__ out, const uint16_t *__restrict__ gate, int64_t gate_ts,
                    int64_t gate_hs, int q_len, int kv_len, int n_q_heads, int n_kv_heads, float scale_log2, int *__restrict__ err, uint32_t launch_id) {
+    constexpr int kTileBytes = T5Shape<D>::kTileBytes;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) T5Bars bars;
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const uint32_t sQ = t5_s32(smem);                       // Q tile 0, Q tile 1
-    const uint32_t sKV = sQ + 2 * kT5TileBytes;             // stage s: K at sKV + 2 s tile, V one tile later
+    const uint32_t sKV = sQ + 2 * kTileBytes;             // stage s: K at sKV + 2 s tile, V one tile later
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int mb = gridDim.x - 1 - blockIdx.x;  // latest (heaviest) query blocks first
     const int h = blockIdx.y, b = blockIdx.z, kvh = h / (n_q_heads / n_kv_heads);
@@ -218,23 +223,23 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     if (warp == 8) {
         // ================================ loader ================================
         if (lane == 0) {
-            t5_expect_tx(t5_s32(&bars.q), 2 * kT5TileBytes);
+            t5_expect_tx(t5_s32(&bars.q), 2 * kTileBytes);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                t5_tma_load(sQ + x * kT5TileBytes, &map_q, 0, h, m0 + x * kT5M, b, t5_s32(&bars.q));
-                t5_tma_load(sQ + x * kT5TileBytes + kT5HalfBytes, &map_q, 64, h, m0 + x * kT5M, b, t5_s32(&bars.q));
+                t5_tma_load(sQ + x * kTileBytes, &map_q, 0, h, m0 + x * kT5M, b, t5_s32(&bars.q));
+                if constexpr (D == 128) t5_tma_load(sQ + x * kTileBytes + kT5HalfBytes, &map_q, 64, h, m0 + x * kT5M, b, t5_s32(&bars.q));
             }
             for (int j = 0; j < n_max && ok; ++j) {
                 const int s = j & 1;
                 if (j >= kT5Stages) ok = t5_wait(t5_s32(&bars.kvempty[s]), ((j >> 1) - 1) & 1, abort_flag);
                 if (!ok) break;
-                const uint32_t sK = sKV + 2 * s * kT5TileBytes, sV = sK + kT5TileBytes;
-                t5_expect_tx(t5_s32(&bars.kfull[s]), kT5TileBytes);
+                const uint32_t sK = sKV + 2 * s * kTileBytes, sV = sK + kTileBytes;
+                t5_expect_tx(t5_s32(&bars.kfull[s]), kTileBytes);
                 t5_tma_load(sK, &map_k, 0, kvh, j * kT5N, b, t5_s32(&bars.kfull[s]));
-                t5_tma_load(sK + kT5HalfBytes, &map_k, 64, kvh, j * kT5N, b, t5_s32(&bars.kfull[s]));
-                t5_expect_tx(t5_s32(&bars.vfull[s]), kT5TileBytes);
+                if constexpr (D == 128) t5_tma_load(sK + kT5HalfBytes, &map_k, 64, kvh, j * kT5N, b, t5_s32(&bars.kfull[s]));
+                t5_expect_tx(t5_s32(&bars.vfull[s]), kTileBytes);
                 t5_tma_load(sV, &map_v, 0, kvh, j * kT5N, b, t5_s32(&bars.vfull[s]));
-                t5_tma_load(sV + kT5HalfBytes, &map_v, 64, kvh, j * kT5N, b, t5_s32(&bars.vfull[s]));
+                if constexpr (D == 128) t5_tma_load(sV + kT5HalfBytes, &map_v, 64, kvh, j * kT5N, b, t5_s32(&bars.vfull[s]));
             }
         }
     } else if (warp == 9) {
@@ -246,14 +251,14 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // and one tile's softmax runs under the other tile's two operations.  The loop is unrolled over the two ring stages, so
         // stage indices, most parities and all descriptor offsets are compile-time constants.
         const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((kT5N >> 3) << 17) | ((kT5M >> 4) << 24);  // bf16 x bf16 -> f32, K-major A and B
-        const uint32_t idesc_pv = idesc_qk | (1u << 16);                                                         // B (V) is MN-major
-        const uint64_t dq0 = t5_desc(sQ, 16, 1024), dk0 = t5_desc(sKV, 16, 1024), dv0 = t5_desc(sKV + kT5TileBytes, kT5HalfBytes, 1024);
+        const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((D >> 3) << 17) | ((kT5M >> 4) << 24);  // B (V) is MN-major
+        const uint64_t dq0 = t5_desc(sQ, 16, 1024), dk0 = t5_desc(sKV, 16, 1024), dv0 = t5_desc(sKV + kTileBytes, kT5HalfBytes, 1024);
         auto issue_s = [&](int x, int st) {  // S^x = Q_x K^T with the K tile of ring stage st
             if (t5_elect()) {
 #pragma unroll
-                for (int ks = 0; ks < kT5D / 16; ++ks) {
+                for (int ks = 0; ks < D / 16; ++ks) {
                     const uint32_t o = (ks >> 2) * kT5HalfBytes + (ks & 3) * 32;
-                    t5_mma_ss(tm + x * kT5N, dq0 + ((x * kT5TileBytes + o) >> 4), dk0 + ((2 * st * kT5TileBytes + o) >> 4), idesc_qk, ks > 0);
+                    t5_mma_ss(tm + x * kT5N, dq0 + ((x * kTileBytes + o) >> 4), dk0 + ((2 * st * kTileBytes + o) >> 4), idesc_qk, ks > 0);
                 }
                 t5_commit(t5_s32(&bars.sfull[x]));
             }
@@ -284,7 +289,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     if (t5_elect()) {
 #pragma unroll
                         for (int ks = 0; ks < kT5N / 16; ++ks)
-                            t5_mma_ts(tm + 256 + x * kT5D, tm + x * kT5N + ks * 8, dv0 + ((2 * i * kT5TileBytes + ks * 2048) >> 4), idesc_pv,
+                            t5_mma_ts(tm + 256 + x * D, tm + x * kT5N + ks * 8, dv0 + ((2 * i * kTileBytes + ks * 2048) >> 4), idesc_pv,
                                       (j > 0 || ks > 0) ? 1u : 0u);
                         t5_commit(t5_s32(&bars.odone[x]));
                         if (last_user) t5_commit(t5_s32(&bars.kvempty[i]));
@@ -307,18 +312,13 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const int x = warp >> 2;  // query tile of this warp group
         const int row = m0 + x * kT5M + (threadIdx.x & 127);
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t tS = tm + lane_base + x * kT5N, tO = tm + lane_base + 256 + x * kT5D;
+        const uint32_t tS = tm + lane_base + x * kT5N, tO = tm + lane_base + 256 + x * D;
         const int nt = n_tiles[x];
         float m_used = -INFINITY, l = 0.0f;
         for (int j = 0; j < nt && ok; ++j) {
             ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.sfull[x]), j & 1, abort_flag));  // warp-uniform: the TMEM
             if (!ok) break;                                                                      // accesses below are warp-collective
             t5_fence_after();
-#ifdef HS_T5_NOSOFTMAX
-            t5_fence_before();
-            t5_arrive(t5_s32(&bars.pready[x]));
-            continue;
-#endif
             const int n0 = j * kT5N;
             const bool masked = n0 + kT5N > min(kv_len, off + m0 + x * kT5M + 1);
             const int lim = min(kv_len - 1, off + row) - n0;  // last visible column of this row inside the tile
@@ -362,7 +362,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     t5_fence_after();
                     const float f = need ? exp2f(m_used - m_new) : 1.0f;
 #pragma unroll
-                    for (int c0 = 0; c0 < kT5D; c0 += 8) {
+                    for (int c0 = 0; c0 < D; c0 += 8) {
                         uint32_t ro[8];
                         t5_ld8(tO + c0, ro);
                         t5_wait_ld();
@@ -424,10 +424,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (ok && nt > 0) {
             t5_fence_after();
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            const int64_t base = ((static_cast<int64_t>(b) * q_len + row) * n_q_heads + h) * kT5D;
+            const int64_t base = ((static_cast<int64_t>(b) * q_len + row) * n_q_heads + h) * D;
             const int64_t gbase = (static_cast<int64_t>(b) * q_len + row) * gate_ts + h * gate_hs;
 #pragma unroll
-            for (int c0 = 0; c0 < kT5D; c0 += 32) {
+            for (int c0 = 0; c0 < D; c0 += 32) {
                 uint32_t r[32];
                 t5_ld32(tO + c0, r);
                 t5_wait_ld();
@@ -851,7 +851,7 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 // [n_seqs, n_tokens, n_heads, head_dim] bf16 -> 4-D map (d, head, token, sequence), box 64 x 1 x box_rows x 1, 128-byte swizzle
-static bool make_map(CUtensorMap *map, const void *base, int n_seqs, int n_tokens, int n_heads, int head_dim = kT5D, int box_rows = kT5N) {
+static bool make_map(CUtensorMap *map, const void *base, int n_seqs, int n_tokens, int n_heads, int head_dim, int box_rows) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[4] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(n_heads), static_cast<cuuint64_t>(n_tokens),
@@ -864,13 +864,40 @@ static bool make_map(CUtensorMap *map, const void *base, int n_seqs, int n_token
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int D>
+static int32_t launch_t5(const uint16_t *q, const uint16_t *k, const uint16_t *v, uint16_t *out, const uint16_t *gate, int64_t gate_ts,
+                         int64_t gate_hs, int n_seqs, int q_len, int kv_len, int n_q_heads, int n_kv_heads, float scale_log2, cudaStream_t s, int *taken) {
+    CUtensorMap mq, mk, mv;
+    if (!make_map(&mq, q, n_seqs, q_len, n_q_heads, D, kT5M) || !make_map(&mk, k, n_seqs, kv_len, n_kv_heads, D, kT5N) ||
+        !make_map(&mv, v, n_seqs, kv_len, n_kv_heads, D, kT5N))
+        return HS_OK;
+    int *err = device_error_word();
+    if (!err) return fail(HS_ERR_DEVICE, "hs_attn_prefill_causal: device error word unavailable");
+    static PerDeviceState configured;
+    const int dev = current_device();
+    if (!configured.get(dev)) {
+        cudaError_t e = cudaFuncSetAttribute(prefill_tc5_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Shape<D>::kSmemBytes);
+        if (e != cudaSuccess) return fail(static_cast<int32_t>(e), "hs_attn_prefill_causal: %s", cudaGetErrorString(e));
+        configured.set(dev, 1);
+    }
+    dim3 grid((q_len + kT5BlockM - 1) / kT5BlockM, n_q_heads, n_seqs);
+    prefill_tc5_kernel<D><<<grid, kT5Threads, T5Shape<D>::kSmemBytes, s>>>(mq, mk, mv, out, gate, gate_ts, gate_hs, q_len, kv_len, n_q_heads, n_kv_heads,
+                                                                          scale_log2, err, next_launch_id());
+    *taken = 1;
+    return HS_OK;
+}
+
 // Returns HS_OK with *taken = 1 when this kernel took the launch, *taken = 0 when the caller should use the
-// mma.sync kernel (head_dim != 128, or no tensor-map encoder in the driver).
+// mma.sync kernel (a single query token, an output that is not
+// 16-byte aligned, or no tensor-map encoder in the driver).
 int32_t prefill_tc5_try(const uint16_t *q, const uint16_t *k, const uint16_t *v, uint16_t *out, const uint16_t *gate, int64_t gate_ts,
                         int64_t gate_hs, int n_seqs, int q_len, int kv_len, int n_q_heads, int n_kv_heads, int head_dim, float scale_log2,
                         cudaStream_t s, int *taken) {
     *taken = 0;
-    if (q_len < 2) return HS_OK;
+    if (q_len < 2 || !aligned(out, 16)) return HS_OK;  // (the epilogue stores 16 bytes at a time)
+    // head_dim 64, all keys in one or two of the mma.sync kernel's tiles: its shorter start wins (32 heads: 4.7 against 6.7 us at 64 keys,
+    // 6.4 against 7.0 at 128, 10.0 against 10.1 at 256; 31.2 against 13.8 at 600)
+    if (head_dim == 64 && kv_len <= 192) return HS_OK;
     if (head_dim == kW5D) {
         CUtensorMap mq, mk, mv;
         if (!make_map(&mq, q, n_seqs, q_len, n_q_heads, kW5D, kW5M) || !make_map(&mk, k, n_seqs, kv_len, n_kv_heads, kW5D, 2 * kW5N) ||
@@ -890,25 +917,8 @@ int32_t prefill_tc5_try(const uint16_t *q, const uint16_t *k, const uint16_t *v,
         *taken = 1;
         return HS_OK;
     }
-    if (head_dim != kT5D) return HS_OK;
-    CUtensorMap mq, mk, mv;
-    if (!make_map(&mq, q, n_seqs, q_len, n_q_heads) || !make_map(&mk, k, n_seqs, kv_len, n_kv_heads) ||
-        !make_map(&mv, v, n_seqs, kv_len, n_kv_heads))
-        return HS_OK;
-    int *err = device_error_word();
-    if (!err) return fail(HS_ERR_DEVICE, "hs_attn_prefill_causal: device error word unavailable");
-    static PerDeviceState configured;
-    const int dev = current_device();
-    if (!configured.get(dev)) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kT5SmemBytes);
-        if (e != cudaSuccess) return fail(static_cast<int32_t>(e), "hs_attn_prefill_causal: %s", cudaGetErrorString(e));
-        configured.set(dev, 1);
-    }
-    dim3 grid((q_len + kT5BlockM - 1) / kT5BlockM, n_q_heads, n_seqs);
-    prefill_tc5_kernel<<<grid, kT5Threads, kT5SmemBytes, s>>>(mq, mk, mv, out, gate, gate_ts, gate_hs, q_len, kv_len, n_q_heads, n_kv_heads, scale_log2, err, next_launch_id());
-    *taken = 1;
-    return HS_OK;
+    return head_dim == 64 ? launch_t5<64>(q, k, v, out, gate, gate_ts, gate_hs, n_seqs, q_len, kv_len, n_q_heads, n_kv_heads, scale_log2, s, taken)
+                          : launch_t5<128>(q, k, v, out, gate, gate_ts, gate_hs, n_seqs, q_len, kv_len, n_q_heads, n_kv_heads, scale_log2, s, taken);
 }
 
 }  // namespace hs
-
