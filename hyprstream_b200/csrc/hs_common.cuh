@@ -104,6 +104,10 @@ struct AppendArgs {
 };
 int32_t kv_write_at_end(const hs_kv_view *view, const void *k_new, const void *v_new, int32_t n_seqs, const int32_t *seq_lens, const void *sin,
                         const void *cos, int32_t rotary_dim, int32_t n_positions, hs_stream_t stream);
+// the host objects' forms, for one sequence: position / length by value instead of in device memory (quant.cu)
+int32_t kv_write_at(const hs_kv_view *view, const void *k_new, const void *v_new, int32_t n_tokens, int32_t start_pos, const void *sin, const void *cos,
+                    int32_t rotary_dim, int32_t n_positions, hs_stream_t stream);
+int32_t kv_gather_len(const hs_kv_view *view, int32_t len, void *k_out, void *v_out, hs_stream_t stream);
 
 // ---- device helpers --------------------------------------------------------------------------
 __device__ __forceinline__ float bf16_bits_to_f32(uint16_t b) { return __uint_as_float(static_cast<uint32_t>(b) << 16); }

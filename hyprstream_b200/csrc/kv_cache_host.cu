@@ -131,6 +131,8 @@ struct hs_pool {
     }
 };
 
+struct hs_view;
+
 // ---- LayerKVCache (kv_cache.rs:1029-1900) ------------------------------------------------------------------
 struct hs_cache {
     hs::Geometry geo;
@@ -142,6 +144,10 @@ struct hs_cache {
     hs_pool *pool = nullptr;    // paged storage
     int64_t owner = 0;
     std::vector<int> blocks;
+    // The cache's own one-sequence view for update() and get(): its pointer table is built when storage was replaced, not on every
+    // call (an allocation, a blocking copy and a free per table and call were most of a small update's time).  Both calls wait for
+    // their stream, so nothing still reads a table that is being replaced.
+    hs_view *own = nullptr;
 
     int page_tokens() const { return pool ? pool->page_tokens : std::max(capacity, 1); }
 
@@ -287,6 +293,30 @@ static int32_t build_view(hs_cache *const *caches, int n, hs_view *out) {
     return HS_OK;
 }
 
+static void drop_view(hs_view *v) {
+    if (!v) return;
+    if (v->table) g_free(v->table);
+    delete v;
+}
+
+// The current one-sequence view of a cache, rebuilt when its storage changed since the last call.
+static int32_t own_view(hs_cache *cache, const hs_kv_view **out) {
+    if (cache->own && (cache->own->generations[0] != cache->generation || cache->own->capacities[0] != cache->capacity)) {
+        drop_view(cache->own);
+        cache->own = nullptr;
+    }
+    if (!cache->own) {
+        hs_view *v = new hs_view();
+        if (int32_t st = build_view(&cache, 1, v)) {
+            delete v;
+            return st;
+        }
+        cache->own = v;
+    }
+    *out = &cache->own->view;
+    return HS_OK;
+}
+
 extern "C" {
 
 int32_t hs_host_set_allocator(hs_alloc_fn alloc_fn, hs_free_fn free_fn) {
@@ -349,6 +379,7 @@ void hs_cache_destroy(hs_cache *cache) {
     cache->release_pages(0);
     cache->slab.release();
     pool_unref(cache->pool);
+    drop_view(cache->own);
     delete cache;
 }
 int32_t hs_cache_reserve(hs_cache *cache, int32_t n_tokens) {
@@ -366,21 +397,12 @@ int32_t hs_cache_update(hs_cache *cache, const void *k_new, const void *v_new, i
                     start_pos, cache->max_seq_len);
     if (n_tokens == 0) return HS_OK;
     if (int32_t st = cache->reserve(end_pos)) return st;
-    hs_view v;
-    hs_cache *one[1] = {cache};
-    if (int32_t st = build_view(one, 1, &v)) return st;
-    int32_t *pos_dev = static_cast<int32_t *>(g_alloc(sizeof(int32_t)));
-    int32_t st = pos_dev ? HS_OK : fail(static_cast<int32_t>(cudaErrorMemoryAllocation), "hs_cache_update: device allocation failed");
-    if (st == HS_OK) {
-        cudaError_t e = cudaMemcpyAsync(pos_dev, &start_pos, sizeof(int32_t), cudaMemcpyHostToDevice, as_stream(stream));
-        if (e != cudaSuccess) st = fail(static_cast<int32_t>(e), "hs_cache_update: %s", cudaGetErrorString(e));
-    }
-    if (st == HS_OK) st = hs_kv_quantize_write(&v.view, k_new, v_new, 1, n_tokens, pos_dev, sin, cos, rotary_dim, n_positions, stream);
-    // the pointer table and the position word must outlive the launch: wait for it before releasing them
+    const hs_kv_view *view = nullptr;
+    if (int32_t st = own_view(cache, &view)) return st;
+    int32_t st = kv_write_at(view, k_new, v_new, n_tokens, start_pos, sin, cos, rotary_dim, n_positions, stream);
+    // the rows are in the cache, and the inputs free to go, when the call returns
     cudaError_t e = cudaStreamSynchronize(as_stream(stream));
     if (st == HS_OK && e != cudaSuccess) st = fail(static_cast<int32_t>(e), "hs_cache_update: %s", cudaGetErrorString(e));
-    if (pos_dev) g_free(pos_dev);
-    if (v.table) g_free(v.table);
     if (st == HS_OK) cache->seq_pos = end_pos;
     return st;
 }
@@ -388,20 +410,11 @@ int32_t hs_cache_update(hs_cache *cache, const void *k_new, const void *v_new, i
 int32_t hs_cache_get(hs_cache *cache, void *k_out, void *v_out, hs_stream_t stream) {
     if (!cache || !k_out || !v_out) return fail(HS_ERR_ARG, "hs_cache_get: bad arguments");
     if (cache->seq_pos == 0) return fail(HS_ERR_CACHE_EMPTY, "Cache is empty");
-    hs_view v;
-    hs_cache *one[1] = {cache};
-    if (int32_t st = build_view(one, 1, &v)) return st;
-    int32_t *len_dev = static_cast<int32_t *>(g_alloc(sizeof(int32_t)));
-    int32_t st = len_dev ? HS_OK : fail(static_cast<int32_t>(cudaErrorMemoryAllocation), "hs_cache_get: device allocation failed");
-    if (st == HS_OK) {
-        cudaError_t e = cudaMemcpyAsync(len_dev, &cache->seq_pos, sizeof(int32_t), cudaMemcpyHostToDevice, as_stream(stream));
-        if (e != cudaSuccess) st = fail(static_cast<int32_t>(e), "hs_cache_get: %s", cudaGetErrorString(e));
-    }
-    if (st == HS_OK) st = hs_kv_gather_dequantize(&v.view, len_dev, 1, cache->seq_pos, k_out, v_out, stream);
+    const hs_kv_view *view = nullptr;
+    if (int32_t st = own_view(cache, &view)) return st;
+    int32_t st = kv_gather_len(view, cache->seq_pos, k_out, v_out, stream);
     cudaError_t e = cudaStreamSynchronize(as_stream(stream));
     if (st == HS_OK && e != cudaSuccess) st = fail(static_cast<int32_t>(e), "hs_cache_get: %s", cudaGetErrorString(e));
-    if (len_dev) g_free(len_dev);
-    if (v.table) g_free(v.table);
     return st;
 }
 
@@ -531,10 +544,6 @@ int32_t hs_view_is_current(const hs_view *view) {
     }
     return HS_OK;
 }
-void hs_view_destroy(hs_view *view) {
-    if (!view) return;
-    if (view->table) g_free(view->table);
-    delete view;
-}
+void hs_view_destroy(hs_view *view) { drop_view(view); }
 
 }  // extern "C"

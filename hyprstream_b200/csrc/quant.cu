@@ -198,7 +198,7 @@ struct KNormArgs {
     float eps;
     int plus_one;         // multiply by (1 + w) instead of w
     uint16_t *k_out;      // optional bf16 [n_seqs, n_tokens, n_kv_heads, head_dim]: the normed, rotated keys
-    int pos_bias;         // added to dst_pos[s]: -1 when the caller hands the attended lengths instead of positions
+    int pos_bias;         // added to dst_pos[s] (or 0): -1 when the caller hands the attended lengths instead of positions
 };
 
 // 8 norm weights, `add` (0 or 1) added to each
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
     constexpr int kUnroll = kWriteElems / E;
     const uint32_t cpr = static_cast<uint32_t>(D) / static_cast<uint32_t>(E);
     const uint32_t total = static_cast<uint32_t>(n_tokens) * static_cast<uint32_t>(H) * cpr;
-    const int base_pos = dst_pos ? dst_pos[s] + kn.pos_bias : 0;
+    const int base_pos = (dst_pos ? dst_pos[s] : 0) + kn.pos_bias;
     void *const *data_pages = is_v ? view.v_pages : view.k_pages;
     void *const *scale_pages = is_v ? view.v_scale_pages : view.k_scale_pages;
     const int tpb = view.block / E;
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kQThreads) kv_gather_kernel(ViewDev view, cons
     const int page_shift = __ffs(view.page_tokens) - 1, h_shift = __ffs(H) - 1;
     const int64_t total = (static_cast<int64_t>(out_tokens) * H) << cpr_shift;
     const int64_t chunk0 = static_cast<int64_t>(blockIdx.x) * (kGatherChunks * kQThreads) + threadIdx.x;
-    const int len = min(seq_lens[s], out_tokens);
+    const int len = seq_lens ? min(seq_lens[s], out_tokens) : out_tokens;
     void *const *data_pages = (is_v ? view.v_pages : view.k_pages) + static_cast<int64_t>(s) * view.pages_per_seq;
     void *const *scale_pages = KIND == HS_KV_BF16 ? nullptr : (is_v ? view.v_scale_pages : view.k_scale_pages) + static_cast<int64_t>(s) * view.pages_per_seq;
     uint4 w[kGatherChunks];
@@ -612,6 +612,12 @@ int32_t hs_kv_quantize_write(const hs_kv_view *view, const void *k_new, const vo
 
 }  // extern "C"
 
+int32_t hs::kv_write_at(const hs_kv_view *view, const void *k_new, const void *v_new, int32_t n_tokens, int32_t start_pos, const void *sin,
+                        const void *cos, int32_t rotary_dim, int32_t n_positions, hs_stream_t stream) {
+    return kv_write_impl("hs_cache_update", view, k_new, v_new, 1, n_tokens, nullptr, sin, cos, rotary_dim, n_positions,
+                         hs::KNormArgs{nullptr, 0.0f, 0, nullptr, start_pos}, stream);
+}
+
 // hs_kv_quantize_write of one new token per sequence at position seq_lens[s] - 1 (used by hs_attn_decode_append when the
 // caller gives no positions and the attention kernel does not take the write itself)
 int32_t hs::kv_write_at_end(const hs_kv_view *view, const void *k_new, const void *v_new, int32_t n_seqs, const int32_t *seq_lens, const void *sin,
@@ -630,27 +636,9 @@ int32_t hs_kv_norm_rope_quantize_write(const hs_kv_view *view, const void *k_pro
                          hs::KNormArgs{k_norm_weight, eps, weight_plus_one, reinterpret_cast<uint16_t *>(k_out), 0}, stream);
 }
 
-int32_t hs_kv_gather_dequantize(const hs_kv_view *view, const int32_t *seq_lens, int32_t n_seqs, int32_t out_tokens,
-                                void *k_out, void *v_out, hs_stream_t stream) {
-    if (int32_t st = check_device()) return st;
-    if (int32_t st = validate_view(view)) return st;
-    if (n_seqs < 0 || out_tokens < 0) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: negative sizes");
-    if (n_seqs == 0 || out_tokens == 0) return HS_OK;
-    if (!seq_lens || !k_out || !v_out) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: NULL pointer");
-    if (!aligned(k_out, 16) || !aligned(v_out, 16)) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: outputs must be 16-byte aligned");
+static int32_t gather_launch(const hs_kv_view *view, const int32_t *seq_lens, int32_t n_seqs, int32_t out_tokens, void *k_out, void *v_out,
+                             hs_stream_t stream) {
     ViewDev d = to_dev(view);
-    if (n_seqs > 32767) {  // the grid's second dimension holds 2 * 32767 rows: the rest in calls of their own
-        const int64_t step = static_cast<int64_t>(32767) * out_tokens * d.n_kv_heads * d.head_dim * 2;
-        hs_kv_view rest = *view;
-        const int64_t pages = static_cast<int64_t>(32767) * view->pages_per_seq;
-        rest.k_pages += pages;
-        rest.v_pages += pages;
-        if (rest.k_scale_pages) rest.k_scale_pages += pages;
-        if (rest.v_scale_pages) rest.v_scale_pages += pages;
-        if (int32_t st = hs_kv_gather_dequantize(view, seq_lens, 32767, out_tokens, k_out, v_out, stream)) return st;
-        return hs_kv_gather_dequantize(&rest, seq_lens + 32767, n_seqs - 32767, out_tokens, static_cast<char *>(k_out) + step,
-                                       static_cast<char *>(v_out) + step, stream);
-    }
     const int64_t chunks = static_cast<int64_t>(out_tokens) * d.n_kv_heads * (d.head_dim / 8);
     dim3 grid(static_cast<unsigned>((chunks + kGatherChunks * kQThreads - 1) / (kGatherChunks * kQThreads)), 2u * static_cast<unsigned>(n_seqs));
     cudaStream_t s = as_stream(stream);
@@ -664,4 +652,34 @@ int32_t hs_kv_gather_dequantize(const hs_kv_view *view, const int32_t *seq_lens,
     return check_launch("hs_kv_gather_dequantize");
 }
 
+int32_t hs_kv_gather_dequantize(const hs_kv_view *view, const int32_t *seq_lens, int32_t n_seqs, int32_t out_tokens,
+                                void *k_out, void *v_out, hs_stream_t stream) {
+    if (int32_t st = check_device()) return st;
+    if (int32_t st = validate_view(view)) return st;
+    if (n_seqs < 0 || out_tokens < 0) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: negative sizes");
+    if (n_seqs == 0 || out_tokens == 0) return HS_OK;
+    if (!seq_lens || !k_out || !v_out) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: NULL pointer");
+    if (!aligned(k_out, 16) || !aligned(v_out, 16)) return fail(HS_ERR_ARG, "hs_kv_gather_dequantize: outputs must be 16-byte aligned");
+    if (n_seqs > 32767) {  // the grid's second dimension holds 2 * 32767 rows: the rest in calls of their own
+        const int64_t step = static_cast<int64_t>(32767) * out_tokens * view->n_kv_heads * view->head_dim * 2;
+        hs_kv_view rest = *view;
+        const int64_t pages = static_cast<int64_t>(32767) * view->pages_per_seq;
+        rest.k_pages += pages;
+        rest.v_pages += pages;
+        if (rest.k_scale_pages) rest.k_scale_pages += pages;
+        if (rest.v_scale_pages) rest.v_scale_pages += pages;
+        if (int32_t st = hs_kv_gather_dequantize(view, seq_lens, 32767, out_tokens, k_out, v_out, stream)) return st;
+        return hs_kv_gather_dequantize(&rest, seq_lens + 32767, n_seqs - 32767, out_tokens, static_cast<char *>(k_out) + step,
+                                       static_cast<char *>(v_out) + step, stream);
+    }
+    return gather_launch(view, seq_lens, n_seqs, out_tokens, k_out, v_out, stream);
+}
+
 }  // extern "C"
+
+int32_t hs::kv_gather_len(const hs_kv_view *view, int32_t len, void *k_out, void *v_out, hs_stream_t stream) {
+    if (int32_t st = check_device()) return st;
+    if (int32_t st = validate_view(view)) return st;
+    if (!aligned(k_out, 16) || !aligned(v_out, 16)) return fail(HS_ERR_ARG, "hs_cache_get: outputs must be 16-byte aligned");
+    return gather_launch(view, nullptr, 1, len, k_out, v_out, stream);
+}
