@@ -1,21 +1,30 @@
 // Causal GQA prefill attention on the 5th-generation tensor cores (bf16; head_dim 128 and 64 first, head_dim 256 further down).
 //
-// One CTA = two 128-row query tiles of one head (256 rows) sharing every K/V tile.  Roles (10 warps):
+// One CTA = two 128-row query tiles of one head (256 rows) sharing every K/V tile.  Keys arrive in tiles of 128 and are worked on
+// in halves of 64 ("steps").  Roles (11 warps):
 //   warp 8  loader: TMA tensor loads (cp.async.bulk.tensor, 128-byte swizzle, no multicast) of the two Q tiles
-//           once and of K/V tiles of 128 keys into a 2-stage shared-memory ring; completion on mbarriers
-//   warp 9  MMA issuer: the warp walks a fixed schedule with one elected lane issuing, per query tile x and key tile j,
-//             S_j = Q_x . K_j^T    (both operands K-major in shared memory, accumulator 128 x 128 fp32 in TMEM)
-//             O_x += P_j . V_j     (P_j read from TMEM as bf16, V_j MN-major in shared memory)
-//           in the order P.V^0_j, S^0_{j+1}, P.V^1_j, S^1_{j+1} (no wait between a P.V and the S that overwrites its P: MMAs
-//           execute in issue order), and tcgen05.commit to the mbarriers that hand results over; one tile's MMAs run
-//           under the other tile's softmax
-//   warps 0-3 / 4-7  softmax of tile 0 / 1: thread = query row (TMEM lane).  Two passes of tcgen05.ld over the
-//           score row (maximum, then exp2 and P as bf16 pairs written back over the scores with tcgen05.st); the
-//           output accumulator in TMEM is rescaled only when a row maximum grew by more than 2^8 (the final
-//           O / l is exact either way); epilogue: O / l, optional sigmoid gate, bf16 store
+//           once and of K/V tiles of 128 keys into two 2-stage shared-memory rings (K and V are released on their own: K as soon as
+//           its last scores exist, a step and a half before V); completion on mbarriers
+//   warps 9, 10  MMA issuers of query tile x = 0, 1: a fixed schedule with one elected lane issuing, per step u,
+//             S_u = Q_x . K_u^T    (both operands K-major in shared memory, accumulator 128 x 64 fp32 in TMEM)
+//             O_x += P_u . V_u     (P_u read from TMEM as bf16, V_u MN-major in shared memory)
+//           in the order P.V_u, S_{u+2} (no wait between a P.V and the S that overwrites its P: MMAs of one thread execute in issue
+//           order), and tcgen05.commit to the mbarriers that hand results over
+//   warps 0-3 / 4-7  softmax of tile 0 / 1: thread = query row (TMEM lane).  The score row goes to registers once (maximum, then
+//           exp2, P as bf16 pairs written back over the scores with tcgen05.st); the output accumulator in TMEM is rescaled only
+//           when a row maximum grew by more than 2^8 (the final O / l is exact either way); epilogue: O / l, optional sigmoid
+//           gate, bf16 store
 //
-// TMEM columns: [0,128) S/P tile 0, [128,256) S/P tile 1, [256,384) O tile 0, [384,512) O tile 1.  Shared
-// memory: 2 x Q 32 KB + 2 x (K 32 KB + V 32 KB).  FLOPs per (query tile, key tile): 2 x 2 x 128^3.
+// Why steps of 64 keys: with one 128-column score buffer per query tile a tile's softmax and its MMAs took turns (clock64 stamps,
+// 128 keys: softmax 1,820 cycles, hand-over 220, P.V + S 1,290 = 3,330 a round, tensor pipe and XU both half idle).  Two 64-column
+// buffers per query tile let S_{u+1} be ready when the softmax of step u ends: 2,720 cycles a round of 128 keys.  What bounds it
+// now: head_dim 128 the shared-memory reads of the 64-column S (A and B, 6 KB per 128 x 64 x 16 MMA: 320 KB a round against 128 B a
+// cycle; 128-column S with one buffer reads 256 KB but takes turns: 10 % slower), head_dim 64 the softmax warps (75 % of the XU).
+// Measured against the one-buffer, one-issuer form (32 / 8 heads): 4 x 8,192 x 128 2.13 -> 1.94 ms = 1.13 PFLOP/s; 1,000 queries
+// behind 3,333 keys 73 -> 67 us; 100 behind 7,900 111 -> 89 us; head_dim 64: 8 x 4,096 1.03 -> 0.87 ms, 2 x 1,531 63 -> 55 us.
+//
+// TMEM columns: S/P of tile x and step u at 128 x + 64 (u & 1), O of tile x at 256 + D x.  Shared memory (D = 128): 2 x Q 32 KB
+// + 2 x (K 32 KB + V 32 KB).  FLOPs per (query tile, step): 2 x 2 x 128 x 64 x D.
 // Bound: tensor pipe (and MUFU exp2).
 //
 // Replaces compute_attention_masked for q_len > 1 (architectures/llama.rs:1023-1119) with GQA expansion
@@ -30,10 +39,10 @@
 
 namespace hs {
 
-constexpr int kT5M = 128, kT5N = 128;
+constexpr int kT5M = 128, kT5N = 128, kT5S = 64;  // query rows of a tile, keys of a K/V tile, keys of a step
 constexpr int kT5Stages = 2;
 constexpr int kT5BlockM = 2 * kT5M;  // two query tiles per CTA
-constexpr int kT5Threads = 320;
+constexpr int kT5Threads = 352;
 constexpr int kT5HalfBytes = kT5N * 128;               // 16 KB: 64 columns of 128 rows, one swizzled box
 template <int D>
 struct T5Shape {                                       // head_dim 128: two boxes a tile; head_dim 64: one
@@ -132,7 +141,7 @@ __device__ __forceinline__ void t5_tma_load(uint32_t dst, const CUtensorMap *map
 }
 
 struct T5Bars {
-    uint64_t q, kfull[kT5Stages], vfull[kT5Stages], kvempty[kT5Stages], sfull[2], pready[2], odone[2];
+    uint64_t q, kfull[kT5Stages], vfull[kT5Stages], kempty[kT5Stages], vempty[kT5Stages], sfull[2][2], pready[2][2], odone[2];
 };
 
 __device__ __forceinline__ uint32_t t5_pack_bf16x2(float lo, float hi) {
@@ -175,7 +184,7 @@ __device__ __forceinline__ float t5_ex2(float x) {
 }
 
 // Two 128-row query tiles (x = 0, 1) per CTA share every K/V tile.  Warps 0-3: softmax of tile 0, warps 4-7: softmax of
-// tile 1, warp 8: loader, warp 9: MMA issuer.  TMEM columns: S/P of tile x at 128x, O of tile x at 256 + 128x.
+// tile 1, warp 8: loader, warps 9 and 10: MMA issuers of tile 0 and 1.
 template <int D>
 __global__ void __launch_bounds__(kT5Threads, 1)
 prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -188,25 +197,29 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     __shared__ int s_abort;
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const uint32_t sQ = t5_s32(smem);                       // Q tile 0, Q tile 1
-    const uint32_t sKV = sQ + 2 * kTileBytes;             // stage s: K at sKV + 2 s tile, V one tile later
+    const uint32_t sKV = sQ + 2 * kTileBytes;               // stage s: K at sKV + 2 s tile, V one tile later
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int mb = gridDim.x - 1 - blockIdx.x;  // latest (heaviest) query blocks first
     const int h = blockIdx.y, b = blockIdx.z, kvh = h / (n_q_heads / n_kv_heads);
     const int m0 = mb * kT5BlockM, off = kv_len - q_len;
-    int n_tiles[2];
+    int n_steps[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         const int lo = m0 + x * kT5M;
-        n_tiles[x] = lo < q_len ? (min(kv_len, off + min(lo + kT5M, q_len)) + kT5N - 1) / kT5N : 0;
+        n_steps[x] = lo < q_len ? (min(kv_len, off + min(lo + kT5M, q_len)) + kT5S - 1) / kT5S : 0;
     }
-    const int n_max = max(n_tiles[0], n_tiles[1]);
+    const int n_max = max(n_steps[0], n_steps[1]), n_kv = (n_max + 1) / 2;  // steps; K/V tiles
     volatile int *abort_flag = &s_abort;
 
     if (threadIdx.x == 0) {
         auto init = [](uint64_t *bar, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(t5_s32(bar)), "r"(count)); };
         init(&bars.q, 1);
-        for (int s = 0; s < kT5Stages; ++s) { init(&bars.kfull[s], 1); init(&bars.vfull[s], 1); init(&bars.kvempty[s], 1); }
-        for (int i = 0; i < 2; ++i) { init(&bars.sfull[i], 1); init(&bars.pready[i], kT5M); init(&bars.odone[i], 1); }
+        const int users = (n_steps[0] > 0) + (n_steps[1] > 0);  // issuers that release a stage (the last tile's release, which nobody waits for, apart)
+        for (int s = 0; s < kT5Stages; ++s) { init(&bars.kfull[s], 1); init(&bars.vfull[s], 1); init(&bars.kempty[s], users); init(&bars.vempty[s], users); }
+        for (int i = 0; i < 2; ++i) {
+            for (int k = 0; k < 2; ++k) { init(&bars.sfull[i][k], 1); init(&bars.pready[i][k], kT5M / 32); }
+            init(&bars.odone[i], 1);
+        }
         s_abort = *reinterpret_cast<volatile uint32_t *>(err + 1) == launch_id ? 1 : 0;  // a time-out recorded by this launch ends its later CTAs at once
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -229,81 +242,87 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 t5_tma_load(sQ + x * kTileBytes, &map_q, 0, h, m0 + x * kT5M, b, t5_s32(&bars.q));
                 if constexpr (D == 128) t5_tma_load(sQ + x * kTileBytes + kT5HalfBytes, &map_q, 64, h, m0 + x * kT5M, b, t5_s32(&bars.q));
             }
-            for (int j = 0; j < n_max && ok; ++j) {
+            for (int j = 0; j < n_kv && ok; ++j) {
                 const int s = j & 1;
-                if (j >= kT5Stages) ok = t5_wait(t5_s32(&bars.kvempty[s]), ((j >> 1) - 1) & 1, abort_flag);
-                if (!ok) break;
                 const uint32_t sK = sKV + 2 * s * kTileBytes, sV = sK + kTileBytes;
+                if (j >= kT5Stages) ok = t5_wait(t5_s32(&bars.kempty[s]), ((j >> 1) - 1) & 1, abort_flag);
+                if (!ok) break;
                 t5_expect_tx(t5_s32(&bars.kfull[s]), kTileBytes);
                 t5_tma_load(sK, &map_k, 0, kvh, j * kT5N, b, t5_s32(&bars.kfull[s]));
                 if constexpr (D == 128) t5_tma_load(sK + kT5HalfBytes, &map_k, 64, kvh, j * kT5N, b, t5_s32(&bars.kfull[s]));
+                if (j >= kT5Stages) ok = t5_wait(t5_s32(&bars.vempty[s]), ((j >> 1) - 1) & 1, abort_flag);
+                if (!ok) break;
                 t5_expect_tx(t5_s32(&bars.vfull[s]), kTileBytes);
                 t5_tma_load(sV, &map_v, 0, kvh, j * kT5N, b, t5_s32(&bars.vfull[s]));
                 if constexpr (D == 128) t5_tma_load(sV + kT5HalfBytes, &map_v, 64, kvh, j * kT5N, b, t5_s32(&bars.vfull[s]));
             }
         }
-    } else if (warp == 9) {
-        // ================================ MMA issuer ================================
-        // The whole warp walks a fixed schedule with blocking waits, and one elected lane issues:
-        //     S^0_0, S^1_0, then per key tile j:  P.V^0_j, S^0_{j+1}, P.V^1_j, S^1_{j+1}
-        // (S^x_j = Q_x K_j^T, 8 MMAs 128x128x16 from shared memory; P.V^x_j: 8 MMAs 128x128x16 with P from tensor memory).  S^x_{j+1}
-        // overwrites the buffer P.V^x_j reads P from: the MMAs of one thread execute in issue order, so nothing waits in between,
-        // and one tile's softmax runs under the other tile's two operations.  The loop is unrolled over the two ring stages, so
-        // stage indices, most parities and all descriptor offsets are compile-time constants.
-        const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((kT5N >> 3) << 17) | ((kT5M >> 4) << 24);  // bf16 x bf16 -> f32, K-major A and B
+    } else if (warp >= 9) {
+        // ================================ MMA issuers ================================
+        // One warp per query tile walks a fixed schedule with blocking waits, and one elected lane issues:
+        //     S_0, S_1, then per step u:  P.V_u, S_{u+2}
+        // (S: D / 16 MMAs 128 x 64 x 16 from shared memory; P.V: 4 MMAs 128 x D x 16 with P from tensor memory).  S_{u+2} overwrites
+        // the scores that P.V_u reads as P: the MMAs of one thread execute in issue order, so nothing waits in between.  The
+        // loops are unrolled over the two ring stages, so stage indices, buffers and all descriptor offsets are compile-time
+        // constants.  (One warp for both tiles spent 220 cycles on each hand-over and was itself what the tiles waited for.)
+        const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((kT5S >> 3) << 17) | ((kT5M >> 4) << 24);  // bf16 x bf16 -> f32, K-major A and B
         const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((D >> 3) << 17) | ((kT5M >> 4) << 24);  // B (V) is MN-major
         const uint64_t dq0 = t5_desc(sQ, 16, 1024), dk0 = t5_desc(sKV, 16, 1024), dv0 = t5_desc(sKV + kTileBytes, kT5HalfBytes, 1024);
-        auto issue_s = [&](int x, int st) {  // S^x = Q_x K^T with the K tile of ring stage st
+        constexpr uint32_t kStepBytes = kT5S * 128;  // 64 rows of a swizzled box
+        const int x = warp - 9, nx = n_steps[x];
+        const uint32_t tS = tm + x * kT5N, tO = tm + 256 + x * D;
+        const uint64_t dq = dq0 + ((x * kTileBytes) >> 4);
+        // S of step u: K tile in ring stage st, half hf of it; releases the K stage behind its last scores
+        auto issue_s = [&](int u, int st, int hf) {
             if (t5_elect()) {
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint32_t o = (ks >> 2) * kT5HalfBytes + (ks & 3) * 32;
-                    t5_mma_ss(tm + x * kT5N, dq0 + ((x * kTileBytes + o) >> 4), dk0 + ((2 * st * kTileBytes + o) >> 4), idesc_qk, ks > 0);
+                    t5_mma_ss(tS + hf * kT5S, dq + (o >> 4), dk0 + ((2 * st * kTileBytes + hf * kStepBytes + o) >> 4), idesc_qk, ks > 0);
                 }
-                t5_commit(t5_s32(&bars.sfull[x]));
+                t5_commit(t5_s32(&bars.sfull[x][hf]));
+                if (hf == 1 || u == nx - 1) t5_commit(t5_s32(&bars.kempty[st]));
             }
             __syncwarp();
         };
-        ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.q), 0, abort_flag) && (n_max == 0 || t5_wait(t5_s32(&bars.kfull[0]), 0, abort_flag)));
-        if (ok) {
+        // O += P.V of step u: V tile in ring stage st, half hf; releases the V stage behind the tile's last P.V
+        auto issue_pv = [&](int u, int st, int hf) {
+            if (t5_elect()) {
+#pragma unroll
+                for (int ks = 0; ks < kT5S / 16; ++ks)
+                    t5_mma_ts(tO, tS + hf * kT5S + ks * 8, dv0 + ((2 * st * kTileBytes + hf * kStepBytes + ks * 2048) >> 4), idesc_pv, (u > 0 || ks > 0) ? 1u : 0u);
+                t5_commit(t5_s32(&bars.odone[x]));
+                if (hf == 1 || u == nx - 1) t5_commit(t5_s32(&bars.vempty[st]));
+            }
+            __syncwarp();
+        };
+        if (nx > 0) ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.q), 0, abort_flag) && t5_wait(t5_s32(&bars.kfull[0]), 0, abort_flag));
+        if (ok && nx > 0) {
             t5_fence_after();
-            if (n_tiles[0] > 0) issue_s(0, 0);
-            if (n_tiles[1] > 0) issue_s(1, 0);
+            issue_s(0, 0, 0);
+            if (nx > 1) issue_s(1, 0, 1);
         }
-        for (int j0 = 0; j0 < n_max && ok; j0 += 2) {
-            const uint32_t p2 = (j0 >> 1) & 1;  // phase parity of the ring stages for tiles j0 and j0 + 1
+        // K/V tile j sits in ring stage j & 1 for the (j >> 1)-th time: parity p for the tiles j0 and j0 + 1
+        for (int j0 = 0; 2 * j0 < nx && ok; j0 += 2) {
+            const uint32_t p = (j0 >> 1) & 1;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int j = j0 + i;
-                if (j >= n_max || !ok) break;
-                // tile j sits in stage i in phase j >> 1 (parity p2); tile j + 1 in stage i ^ 1, in phase (j + 1) >> 1 = parity p2 ^ i
-                bool k_next_ready = false;
+                const int u0 = 2 * (j0 + i);  // the tile's first step
+                if (u0 >= nx || !ok) break;
+                // this tile's V and the next one's K (stage i ^ 1, parity p ^ i): there long before the first P, so waited for first
+                ok = t5_wait(t5_s32(&bars.vfull[i]), p, abort_flag);
+                if (ok && u0 + 2 < nx) ok = t5_wait(t5_s32(&bars.kfull[i ^ 1]), p ^ i, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
 #pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    if (j >= n_tiles[x]) continue;
-                    ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.pready[x]), i, abort_flag) &&
-                                                     t5_wait(t5_s32(&bars.vfull[i]), p2, abort_flag));
+                for (int hf = 0; hf < 2; ++hf) {
+                    if (u0 + hf >= nx || !ok) continue;
+                    // P of the step is written (buffer hf for the u0 / 2-th time)
+                    ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.pready[x][hf]), i, abort_flag));
                     if (!ok) break;
                     t5_fence_after();
-                    const bool last_user = x == 1 || j >= n_tiles[1];  // the stage of tile j is free once this P.V has completed
-                    if (t5_elect()) {
-#pragma unroll
-                        for (int ks = 0; ks < kT5N / 16; ++ks)
-                            t5_mma_ts(tm + 256 + x * D, tm + x * kT5N + ks * 8, dv0 + ((2 * i * kTileBytes + ks * 2048) >> 4), idesc_pv,
-                                      (j > 0 || ks > 0) ? 1u : 0u);
-                        t5_commit(t5_s32(&bars.odone[x]));
-                        if (last_user) t5_commit(t5_s32(&bars.kvempty[i]));
-                    }
-                    __syncwarp();
-                    if (j + 1 < n_tiles[x]) {
-                        if (!k_next_ready) {
-                            ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.kfull[i ^ 1]), p2 ^ i, abort_flag));
-                            if (!ok) break;
-                            t5_fence_after();
-                            k_next_ready = true;
-                        }
-                        issue_s(x, i ^ 1);
-                    }
+                    issue_pv(u0 + hf, i, hf);
+                    if (u0 + hf + 2 < nx) issue_s(u0 + hf + 2, i ^ 1, hf);
                 }
             }
         }
@@ -312,27 +331,27 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const int x = warp >> 2;  // query tile of this warp group
         const int row = m0 + x * kT5M + (threadIdx.x & 127);
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t tS = tm + lane_base + x * kT5N, tO = tm + lane_base + 256 + x * D;
-        const int nt = n_tiles[x];
+        const uint32_t tO = tm + lane_base + 256 + x * D;
+        const int nt = n_steps[x];
         float m_used = -INFINITY, l = 0.0f;
-        for (int j = 0; j < nt && ok; ++j) {
-            ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.sfull[x]), j & 1, abort_flag));  // warp-uniform: the TMEM
-            if (!ok) break;                                                                      // accesses below are warp-collective
+        for (int u = 0; u < nt && ok; ++u) {
+            ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.sfull[x][u & 1]), (u >> 1) & 1, abort_flag));  // warp-uniform: the TMEM
+            if (!ok) break;                                                                                    // accesses below are warp-collective
             t5_fence_after();
-            const int n0 = j * kT5N;
-            const bool masked = n0 + kT5N > min(kv_len, off + m0 + x * kT5M + 1);
-            const int lim = min(kv_len - 1, off + row) - n0;  // last visible column of this row inside the tile
-            // ---- pass 1: row maximum (all four loads in flight, one wait) ----
+            const uint32_t tS = tm + lane_base + x * kT5N + (u & 1) * kT5S;
+            const int n0 = u * kT5S;
+            const bool masked = n0 + kT5S > min(kv_len, off + m0 + x * kT5M + 1);
+            const int lim = min(kv_len - 1, off + row) - n0;  // last visible column of this row inside the step
+            // ---- row maximum (the score row stays in registers for the exponentials: one trip to tensor memory) ----
             float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-            // (the score row stays in registers for the second pass: one trip to tensor memory per tile and row)
-            uint32_t r[4][32];
+            uint32_t r[2][32];
             {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) t5_ld32(tS + 32 * c, r[c]);
+                for (int c = 0; c < 2; ++c) t5_ld32(tS + 32 * c, r[c]);
                 t5_wait_ld();
                 if (!masked) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < 2; ++c)
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
                             mx0 = t5_max3(mx0, __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
@@ -342,7 +361,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                         }
                 } else {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < 2; ++c)
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
                             const float a0 = 32 * c + i > lim ? -INFINITY : __uint_as_float(r[c][i]);
@@ -352,12 +371,12 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 }
             }
             const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * scale_log2);
-            if (j == 0) {
+            if (u == 0) {
                 m_used = m_new;
             } else {
                 const bool need = m_new - m_used > kT5RescaleThreshold;  // false while both are -inf (NaN compares false)
                 if (__any_sync(0xffffffffu, need)) {
-                    ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x]), (j - 1) & 1, abort_flag));
+                    ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x]), (u - 1) & 1, abort_flag));
                     if (!ok) break;
                     t5_fence_after();
                     const float f = need ? exp2f(m_used - m_new) : 1.0f;
@@ -376,50 +395,51 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 }
                 if (m_used == -INFINITY) m_used = m_new;
             }
-            // ---- pass 2: P = exp2(s * scale - m) as bf16 pairs, written over the score buffer ----
+            // ---- P = exp2(s * scale - m) as bf16 pairs, written over the score buffer ----
             const float neg_m = m_used == -INFINITY ? 0.0f : -m_used;
             float ps0 = 0.0f, ps1 = 0.0f;
-            {
-                if (!masked) {
-                    const uint64_t sc2 = t5_pack2(scale_log2, scale_log2), nm2 = t5_pack2(neg_m, neg_m);
-                    uint64_t acc_a = t5_pack2(0.0f, 0.0f), acc_b = acc_a;
+            if (!masked) {
+                const uint64_t sc2 = t5_pack2(scale_log2, scale_log2), nm2 = t5_pack2(neg_m, neg_m);
+                uint64_t acc_a = t5_pack2(0.0f, 0.0f), acc_b = acc_a;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t w[16];
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t w[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            float x0, x1;
-                            t5_unpack2(t5_fma2(t5_pack2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), sc2, nm2), x0, x1);
-                            const float p0 = t5_ex2(x0), p1 = t5_ex2(x1);
-                            if (i & 1) acc_b = t5_add2(acc_b, t5_pack2(p0, p1)); else acc_a = t5_add2(acc_a, t5_pack2(p0, p1));
-                            w[i] = t5_pack_bf16x2(p0, p1);
-                        }
-                        t5_st16(tS + 16 * c, w);
+                    for (int i = 0; i < 16; ++i) {
+                        float x0, x1;
+                        t5_unpack2(t5_fma2(t5_pack2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), sc2, nm2), x0, x1);
+                        const float p0 = t5_ex2(x0), p1 = t5_ex2(x1);
+                        if (i & 1) acc_b = t5_add2(acc_b, t5_pack2(p0, p1)); else acc_a = t5_add2(acc_a, t5_pack2(p0, p1));
+                        w[i] = t5_pack_bf16x2(p0, p1);
                     }
-                    float a0, a1;
-                    t5_unpack2(t5_add2(acc_a, acc_b), a0, a1);
-                    ps0 = a0; ps1 = a1;
-                } else {
+                    t5_st16(tS + 16 * c, w);
+                }
+                float a0, a1;
+                t5_unpack2(t5_add2(acc_a, acc_b), a0, a1);
+                ps0 = a0; ps1 = a1;
+            } else {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t w[16];
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t w[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float p0 = 32 * c + 2 * i > lim ? 0.0f : t5_ex2(fmaf(__uint_as_float(r[c][2 * i]), scale_log2, neg_m));
-                            const float p1 = 32 * c + 2 * i + 1 > lim ? 0.0f : t5_ex2(fmaf(__uint_as_float(r[c][2 * i + 1]), scale_log2, neg_m));
-                            ps0 += p0; ps1 += p1;
-                            w[i] = t5_pack_bf16x2(p0, p1);
-                        }
-                        t5_st16(tS + 16 * c, w);
+                    for (int i = 0; i < 16; ++i) {
+                        const float p0 = 32 * c + 2 * i > lim ? 0.0f : t5_ex2(fmaf(__uint_as_float(r[c][2 * i]), scale_log2, neg_m));
+                        const float p1 = 32 * c + 2 * i + 1 > lim ? 0.0f : t5_ex2(fmaf(__uint_as_float(r[c][2 * i + 1]), scale_log2, neg_m));
+                        ps0 += p0; ps1 += p1;
+                        w[i] = t5_pack_bf16x2(p0, p1);
                     }
+                    t5_st16(tS + 16 * c, w);
                 }
             }
             l += ps0 + ps1;
             t5_wait_st();
             t5_fence_before();
-            t5_arrive(t5_s32(&bars.pready[x]));
+            __syncwarp();  // the warp's 32 rows of P are written: one arrival for all of them
+            if (lane == 0) t5_arrive(t5_s32(&bars.pready[x][u & 1]));
         }
         // ---- epilogue ----
+        // (the last scores prove P.V_{nt-3} complete, no more: the parity of step nt - 1 can be told only once step nt - 2 is in)
+        if (ok && nt > 1) ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x]), (nt - 2) & 1, abort_flag));
         if (ok && nt > 0) ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x]), (nt - 1) & 1, abort_flag));
         if (ok && nt > 0) {
             t5_fence_after();
