@@ -1,10 +1,11 @@
-"""GPU: the tensor-core decode kernel over bf16 caches, for every head_dim and query group it serves, at the edges of its
-16-token tiles, of its CTA ranges and of pages that are no multiple of a tile."""
+"""GPU: the tensor-core decode kernel for every kind, head_dim, scale block and query group it serves, at the edges of its 16-token
+tiles, of its CTA ranges and of pages that are no multiple of a tile; and code pages that are aligned to words only."""
 import math
 
 import pytest
 import torch
 
+from oracle import quant_ref as qr
 from tests.util import no_device_error
 
 pytestmark = pytest.mark.gpu
@@ -19,21 +20,33 @@ def _attend64(q, k, v):
     return torch.einsum("hl,lhd->hd", p, vv)
 
 
-def _run(cuda, hq, hkv, d, lens, page_tokens, seed, edit=None):
+def _stored(t, kind, block, sdt):
+    """t as a cache of this kind holds it, in float64."""
+    codes, amax = qr.quantize(t.float().numpy(), kind, block, bool(sdt))
+    idx = torch.from_numpy(codes).long()
+    if kind != 1:
+        idx = torch.stack((idx >> 4, idx & 15), 1).flatten()
+    book = torch.from_numpy(qr.codebook(kind)).double()
+    return (book[idx].view(-1, block) * torch.from_numpy(amax.astype("float64"))[:, None]).view(t.shape)
+
+
+def _run(cuda, hq, hkv, d, lens, page_tokens, seed, edit=None, kind=0, block=64, sdt=0):
     from hyprstream_b200 import kv_cache as kc
     from hyprstream_b200 import ops
 
     g = torch.Generator().manual_seed(seed)
-    pool = kc.BlockPool(sum((l + page_tokens - 1) // page_tokens for l in lens) + 1, hkv, d, cuda, kind=0, page_tokens=page_tokens) if page_tokens else None
+    pool = kc.BlockPool(sum((l + page_tokens - 1) // page_tokens for l in lens) + 1, hkv, d, cuda, kind=kind, block=block, scale_dtype=sdt,
+                        page_tokens=page_tokens) if page_tokens else None
     caches, kvs = [], []
     for i, l in enumerate(lens):
         k, v = (torch.randn(1, l, hkv, d, generator=g).bfloat16() for _ in range(2))
         if edit:
             edit(k, v)
-        c = kc.LayerKVCache.new_paged(1 << 20, pool, owner=i) if pool else kc.LayerKVCache(1 << 20, kc.KVQuantType.NONE, hkv, d, cuda)
+        c = kc.LayerKVCache.new_paged(1 << 20, pool, owner=i) if pool else kc.LayerKVCache(
+            1 << 20, kc.KVQuantType(kind), hkv, d, cuda, block=block, scale_dtype=sdt)
         c.update(k.to(cuda), v.to(cuda), 0)
         caches.append(c)
-        kvs.append((k[0], v[0]))
+        kvs.append((k[0], v[0]) if kind == 0 else tuple(_stored(t, kind, block, sdt) for t in (k[0], v[0])))
     q = torch.randn(len(lens), hq, d, generator=g).bfloat16()
     view, keep = kc.make_view(caches)
     out = ops.decode_attention(q.to(cuda), view, torch.tensor(lens, dtype=torch.int32, device=cuda))
@@ -64,3 +77,47 @@ def test_bf16_decode_infinite_value(cuda, g):
     o = out[0].float().view(2, g, 128)
     assert (o[0, :, 5] == math.inf).all() and (o[1, :, 9] == -math.inf).all()
     assert torch.isfinite(o).sum().item() == o.numel() - 2 * g
+
+
+@pytest.mark.parametrize("kind", [1, 2, 3])
+@pytest.mark.parametrize("d,block,sdt", [(64, 64, 0), (64, 64, 1), (128, 64, 0), (128, 128, 1), (256, 64, 1), (256, 128, 0), (256, 256, 0)])
+@pytest.mark.parametrize("g", [1, 2, 4, 8])
+@pytest.mark.parametrize("hkv,lens,page_tokens", [(2, [1, 15, 17, 33, 300, 1000], 0), (3, [5, 48, 39, 41, 700], 40)])
+def test_code_decode_every_shape(cuda, kind, d, block, sdt, g, hkv, lens, page_tokens):
+    q, kvs, out = _run(cuda, hkv * g, hkv, d, lens, page_tokens, seed=d + g + kind, kind=kind, block=block, sdt=sdt)
+    # the int8 kernel for 2 x 256 heads (group 8, blocks of 64 and 128) holds P in fp16, whose small values are coarser
+    fp16_p = (kind, d, g, hkv) == (1, 256, 8, 2) and block < 256
+    for r, (k, v) in enumerate(kvs):
+        ref = _attend64(q[r], k, v)
+        err = (out[r].double() - ref).abs()
+        # one rounding to bf16 (2^-9 of the value) on top of probabilities and table values that carry 16 bits
+        assert (err <= ref.abs() * 2.0 ** -8 + (4e-3 if fp16_p else 5e-4)).all(), (lens[r], err.max().item())
+    no_device_error()
+
+
+@pytest.mark.parametrize("kind,d,g", [(1, 64, 4), (2, 128, 2), (3, 64, 8)])
+@pytest.mark.parametrize("shift", [4, 8])
+def test_pages_aligned_to_words(cuda, kind, d, g, shift):
+    """Code pages at an address that is a multiple of 4 (8) bytes only give what aligned ones give, bit for bit."""
+    from hyprstream_b200 import ffi, ops
+
+    n, hkv, page = 150, 2, 160
+    row = (d if kind == 1 else d // 2) * hkv
+    gen = torch.Generator().manual_seed(d)
+    kv = [torch.randint(0, 256, (page * row,), generator=gen).to(torch.uint8).to(cuda) for _ in range(2)]
+    scales = [(torch.rand(page * hkv * (d // 64), generator=gen) + 0.5).to(cuda) for _ in range(2)]
+    q = torch.randn(1, hkv * g, d, generator=gen).bfloat16().to(cuda)
+    outs = []
+    for by in (0, shift):
+        bufs = []
+        for t in kv:
+            b = torch.zeros(t.numel() + 64, dtype=torch.uint8, device=cuda)
+            b[by:by + t.numel()] = t
+            bufs.append(b)
+        tabs = [torch.tensor([p], dtype=torch.int64, device=cuda) for p in (bufs[0].data_ptr() + by, bufs[1].data_ptr() + by,
+                                                                            scales[0].data_ptr(), scales[1].data_ptr())]
+        view = ffi.KVView(kind, ffi.SCALE_F32, 64, hkv, d, page, 1, 0, *[t.data_ptr() for t in tabs])
+        outs.append(ops.decode_attention(q, view, torch.tensor([n], dtype=torch.int32, device=cuda)))
+        torch.cuda.synchronize()
+    assert torch.equal(outs[0], outs[1])
+    no_device_error()
