@@ -33,16 +33,19 @@ struct MmLayout {
     static constexpr int kTileBytes = kScaleOff + (kQuant ? 2 * kMmTile * (D / 64) * 4 : 0);
     // bytes in flight: 6.5 TB/s / 148 SMs at ~1 us is ~44 KB per SM; the rings of an SM hold 100-190 KB (32-64 KB for the small
     // rows of head_dim 64).  At least three stages: a tile's scales are parked one fetch after its rows.
-    static constexpr int kStages = kTileBytes >= 8192 || (D == 256 && kRow == 128) ? 3 : (kTileBytes >= 4096 ? 4 : 5);
+    static constexpr int kStages = kTileBytes >= 4096 ? 3 : 5;
     static constexpr int kORow = D + 4;                 // floats between the heads of a warp's merge rows (bank spread)
     static constexpr int kMergeOff = kMmWarps * kStages * kTileBytes;
     static constexpr int kMlOff = kMergeOff + kMmWarps * G * kORow * 4;
-    // 4-bit kinds: uint2 [256][kLutCols], code byte -> both values as bf16 pairs (upper terms, lower terms).  16 columns make the
-    // 8-byte lookups of a half warp free of bank conflicts; head_dim 256 has 8 (two lanes a column), so that two CTAs fit an SM
-    static constexpr int kLutCols = D == 256 ? 8 : 16;
+    // 4-bit kinds: uint2 [256][kLutCols], code byte -> both values as bf16 pairs (upper terms, lower terms).  8 columns, two
+    // lanes of a half warp each (16 would be free of bank conflicts and cost a CTA per SM)
+    static constexpr int kLutCols = 8;
     static constexpr int kLutOff = (kMlOff + kMmWarps * G * 2 * 4 + 127) / 128 * 128;
     static constexpr int kTotal = kLutOff + (kQuant && KIND != HS_KV_INT8 ? 256 * kLutCols * 8 : 0);
-    static constexpr int kCtasPerSm = 2 * (kTotal + 1024) <= 228 * 1024 ? 2 : 1;
+    // codes take several times the instructions per byte that bf16 rows take: as many warps as the registers allow (a warp's chain
+    // of lookups, MMAs and shuffles is latency, not throughput)
+    static constexpr int kWant = !kQuant || D == 256 || G == 8 ? 2 : (D == 128 ? 3 : 4);
+    static constexpr int kCtasPerSm = kWant * (kTotal + 1024) <= 228 * 1024 ? kWant : (2 * (kTotal + 1024) <= 228 * 1024 ? 2 : 1);
     static_assert(kTotal + 1024 <= 228 * 1024, "a CTA must fit its SM's shared memory");
     // 16-byte chunk c of token row t sits at chunk c ^ swz(t).  bf16: ldmatrix reads 8 rows at one chunk.  u8 and 4-bit codes: a
     // K read takes 4 (2) chunks of neighbouring rows, a V read 2 (1) chunks of every other row.
