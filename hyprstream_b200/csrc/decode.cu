@@ -133,7 +133,7 @@ int32_t decode_int8_tc_try(const ViewDev &v, const uint16_t *q, const int32_t *s
 
 // decode_mma.cu: tensor-core kernel for every kind, head_dim and query group
 int32_t decode_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
-                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, cudaStream_t s);
+                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, const AppendArgs &ap, cudaStream_t s);
 
 // ---- decode scratch that lives inside the library ------------------------------------------------
 // Backing store of hs_attn_decode_static(): the split-KV partials go here instead of into a workspace the
@@ -229,11 +229,11 @@ int32_t hs::decode_impl(const void *q, const hs_kv_view *view, const int32_t *se
     prof_begin(s);
     st = decode_int8_tc_try(v, qp, seq_lens, n_seqs, n_q_heads, softmax_scale, o_part, lse_part, err, s, &tc_ctas,
                             reinterpret_cast<uint16_t *>(out), reinterpret_cast<const uint16_t *>(gate), o_shard, lse_shard, &merged, shard, after_write, append);
-    if (st == HS_OK && append && tc_ctas == 0) {  // the tensor-core kernel did not take the launch: nothing was written, the caller writes
+    if (st == HS_OK && append && tc_ctas == 0 && view->kind != HS_KV_BF16) {  // no kernel writes these codes itself: nothing was written, the caller writes
         prof_end(s);
         return HS_OK;
     }
-    if (appended && append && tc_ctas > 0) *appended = 1;
+    if (appended && append) *appended = 1;
     if (st == HS_OK && shard && tc_ctas == 0) {
         prof_end(s);
         return fail(HS_ERR_UNSUPPORTED, "hs_attn_decode_sharded: only the tensor-core decode kernel exchanges shard results (quantised cache, 8 kv heads x 128 "
@@ -241,7 +241,7 @@ int32_t hs::decode_impl(const void *q, const hs_kv_view *view, const int32_t *se
                                         "all-gather and hs_attn_merge_partials_strided for this shape");
     }
     if (st == HS_OK && tc_ctas == 0) {
-        st = decode_mma(v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, decode_max_ctas(), &n_ctas, &tile, after_write != 0, s);
+        st = decode_mma(v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, decode_max_ctas(), &n_ctas, &tile, after_write != 0, append ? *append : AppendArgs{}, s);
     }
     prof_end(s);
     if (st != HS_OK) return st;
@@ -318,14 +318,14 @@ int32_t hs_attn_decode_append(const void *q, const void *k_new, const void *v_ne
     if (!k_new || !v_new) return fail(HS_ERR_ARG, "hs_attn_decode_append: NULL new token");
     if (dst_pos == nullptr) {
         // the new token goes to position seq_lens[s] - 1: the attention kernel can write it itself (u8 caches on the tensor-core
-        // kernel: one launch per step); otherwise the write kernel runs first, at those positions
+        // kernel, bf16 caches); otherwise the write kernel runs first, at those positions
         if (!aligned(k_new, 16) || !aligned(v_new, 16)) return fail(HS_ERR_ARG, "hs_attn_decode_append: inputs must be 16-byte aligned");
         if (sin != nullptr && (!cos || rotary_dim <= 0 || rotary_dim % 16 != 0 || (view && rotary_dim > view->head_dim) || n_positions <= 0))
             return fail(HS_ERR_UNSUPPORTED, "hs_attn_decode_append: rotary_dim must be a positive multiple of 16 <= head_dim");
         AppendArgs ap{reinterpret_cast<const uint16_t *>(k_new), reinterpret_cast<const uint16_t *>(v_new), reinterpret_cast<const uint16_t *>(sin),
                       reinterpret_cast<const uint16_t *>(cos), rotary_dim, n_positions};
         int appended = 0;
-        if (view && view->kind == HS_KV_INT8) {
+        if (view && (view->kind == HS_KV_INT8 || (view->kind == HS_KV_BF16 && n_seqs <= 32767))) {  // (more sequences: refused by the write)
             if (int32_t st = decode_impl(q, view, seq_lens, n_seqs, n_q_heads, softmax_scale, out, gate, workspace, workspace_bytes, nullptr, nullptr,
                                          nullptr, stream, 0, &ap, &appended))
                 return st;

@@ -16,6 +16,7 @@
 // Measured against the CUDA-core form (a cold launch by itself), bf16, 32 / 8 heads x 128: 16 paged sequences of 100 to 6,000 tokens
 // (247 MB) 150 -> 44.0 us = 5.6 TB/s; one sequence of 4,096 tokens 23.3 -> 9.3 us.
 #include "hs_common.cuh"
+#include "quant_dev.cuh"
 
 namespace hs {
 
@@ -103,7 +104,7 @@ __device__ __forceinline__ uint2 lut_pairs(uint32_t lut, uint32_t w, uint32_t k)
 template <int KIND, int D, int G>
 __global__ void __launch_bounds__(kMmThreads, MmLayout<KIND, D, G>::kCtasPerSm)
 decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *__restrict__ seq_lens, int n_seqs, int n_q_heads,
-                  float scale_log2, float *__restrict__ o_part, float *__restrict__ lse_part, int *__restrict__ err) {
+                  float scale_log2, float *__restrict__ o_part, float *__restrict__ lse_part, int *__restrict__ err, AppendArgs ap) {
     using LT = MmLayout<KIND, D, G>;
     constexpr bool kQuant = LT::kQuant, kFour = kQuant && KIND != HS_KV_INT8;
     constexpr int kChunks = LT::kChunks;           // 16-byte chunks of a row
@@ -119,13 +120,15 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
 
     // ---- the CTA's range of the concatenated tile list (every warp for itself, 32 lengths per load) ----
     int64_t total = 0;
-    bool over = false;
+    bool over = false, unwritable = false;
     for (int base = 0; base < n_seqs; base += 32) {
         const int L = base + lane < n_seqs ? seq_lens[base + lane] : 0;
         over |= L > cap;
+        unwritable |= base + lane < n_seqs && (L > cap || L <= 0);  // no place for a new token at L - 1
         total += __reduce_add_sync(0xffffffffu, static_cast<unsigned>(tiles_of(L)));
     }
     if (over && warp == 0 && cta == 0 && kvh == 0) atomicOr(err, HS_DEVERR_DECODE_RANGE);
+    if (!kQuant && ap.k_new != nullptr && unwritable && warp == 0 && cta == 0 && kvh == 0) atomicOr(err, HS_DEVERR_KV_WRITE_RANGE);
     // never more working CTAs than tiles (the merge uses the same rule)
     const int64_t n_ctas = total < static_cast<int64_t>(gridDim.x) ? (total > 0 ? total : 1) : static_cast<int64_t>(gridDim.x);
     if (cta >= n_ctas) return;
@@ -198,6 +201,32 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
             const unsigned char *k0 = reinterpret_cast<const unsigned char *>(kp[page0]), *v0 = reinterpret_cast<const unsigned char *>(vp[page0]);
             constexpr int kPer = kMmTile * kChunks / 32, kRows = 32 / kChunks;  // copies per lane and operand; rows the warp covers per copy
             const int row0 = lane / kChunks, c = lane % kChunks;
+            // The step's new token (bf16 caches; LayerKVCache::update in the same launch, kv_cache.rs:1275-1496): the warp that fetches a
+            // sequence's last tile takes the token's K (rotated) and V row of its kv head from the inputs, writes them to the cache -
+            // the bits the write kernel writes - and puts them into the ring in place of a copy.  A position past the rotation
+            // table is recorded and its K row left as it is, as the write kernel does.
+            int k_row = -1, v_row = -1;  // rows of this tile that do not come from the cache
+            if constexpr (!kQuant) {
+                const int pos = f_len - 1;
+                if (ap.k_new != nullptr && pos - t0 < kMmTile && seq_lens[f_r] <= cap) {
+                    v_row = pos - t0;
+                    const bool in_table = ap.sin == nullptr || pos < ap.n_positions;
+                    if (in_table) k_row = v_row;
+                    else if (lane == 0) atomicOr(err, HS_DEVERR_KV_WRITE_RANGE);
+                    const int page = view.pages_per_seq == 1 ? 0 : pos / view.page_tokens;
+                    const int64_t at = (static_cast<int64_t>(pos - page * view.page_tokens) * H + kvh) * LT::kRow;
+                    const int64_t src = (static_cast<int64_t>(f_r) * H + kvh) * D;
+                    for (int i = lane; i < 2 * kChunks; i += 32) {
+                        const bool is_v = i >= kChunks;
+                        const int ch = is_v ? i - kChunks : i;
+                        if (!is_v && !in_table) continue;
+                        const uint4 w = row8_rope((is_v ? ap.v_new : ap.k_new) + src, ch * 8, is_v ? nullptr : ap.sin, ap.cos, pos, ap.rotary_dim);
+                        *reinterpret_cast<uint4 *>(static_cast<unsigned char *>((is_v ? vp : kp)[page]) + at + ch * 16) = w;
+                        *reinterpret_cast<uint4 *>(ring_ptr + f_stage * LT::kTileBytes + (is_v ? kMmTile * LT::kRow : 0) + v_row * LT::kRow +
+                                                   ((ch ^ LT::swz(v_row)) << 4)) = w;
+                    }
+                }
+            }
             const bool fast = whole_pages && (!kQuant || ((reinterpret_cast<uintptr_t>(k0) | reinterpret_cast<uintptr_t>(v0)) & 15u) == 0);
             if (fast) {
                 const int64_t off = (static_cast<int64_t>(t0 - page0 * view.page_tokens + row0) * H + kvh) * LT::kRow + c * 16;
@@ -208,8 +237,8 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
                     const int row = i * kRows + row0;
                     const bool live = t0 + row < f_len;
                     const uint32_t dst = sK + row * LT::kRow + ((c ^ LT::swz(row)) << 4);
-                    mm_cp16(dst, live ? ka : k0, live ? 16 : 0);
-                    mm_cp16(dst + kMmTile * LT::kRow, live ? va : v0, live ? 16 : 0);
+                    if (kQuant || row != k_row) mm_cp16(dst, live ? ka : k0, live ? 16 : 0);
+                    if (kQuant || row != v_row) mm_cp16(dst + kMmTile * LT::kRow, live ? va : v0, live ? 16 : 0);
                 }
             } else {
 #pragma unroll 1
@@ -221,8 +250,8 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
                     const uint32_t dst = sK + row * LT::kRow + ((c ^ LT::swz(row)) << 4);
                     const unsigned char *ka = reinterpret_cast<const unsigned char *>(kp[page]) + off, *va = reinterpret_cast<const unsigned char *>(vp[page]) + off;
                     if (!kQuant || ((reinterpret_cast<uintptr_t>(ka) | reinterpret_cast<uintptr_t>(va)) & 15u) == 0) {
-                        mm_cp16(dst, ka, live ? 16 : 0);
-                        mm_cp16(dst + kMmTile * LT::kRow, va, live ? 16 : 0);
+                        if (kQuant || row != k_row) mm_cp16(dst, ka, live ? 16 : 0);
+                        if (kQuant || row != v_row) mm_cp16(dst + kMmTile * LT::kRow, va, live ? 16 : 0);
                     } else {  // pages of codes that are aligned to words only
                         for (int b = 0; b < 16; b += 4) {
                             mm_cp4(dst + b, ka + b, live ? 4 : 0);
@@ -513,7 +542,7 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
 
 template <int KIND, int D, int G>
 static int32_t launch_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
-                          float *lse_part, int *err, int max_ctas, int *n_ctas_out, bool after_write, cudaStream_t s) {
+                          float *lse_part, int *err, int max_ctas, int *n_ctas_out, bool after_write, const AppendArgs &ap, cudaStream_t s) {
     using LT = MmLayout<KIND, D, G>;
     auto kern = decode_mma_kernel<KIND, D, G>;
     static PerDeviceState configured;
@@ -536,7 +565,7 @@ static int32_t launch_mma(const ViewDev &v, const uint16_t *q, const int32_t *se
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = after_write ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, v, q, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, v, q, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, ap);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(static_cast<int32_t>(e), "hs_attn_decode: %s", cudaGetErrorString(e));
@@ -544,12 +573,12 @@ static int32_t launch_mma(const ViewDev &v, const uint16_t *q, const int32_t *se
     return HS_OK;
 }
 
-// *n_ctas_out = CTAs per kv head, *tile_out = tokens per tile, as the merge kernel needs them.
+// `ap` (bf16 caches only, else k_new == NULL): the step's new tokens.  *n_ctas_out = CTAs per kv head, *tile_out = tokens per tile, as the merge kernel needs them.
 int32_t decode_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
-                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, cudaStream_t s) {
+                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, const AppendArgs &ap, cudaStream_t s) {
     *tile_out = kMmTile;
     const int G = n_q_heads / v.n_kv_heads;
-#define HS_MMA_RUN(K, DD, GG) launch_mma<K, DD, GG>(v, q, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, max_ctas, n_ctas_out, after_write, s)
+#define HS_MMA_RUN(K, DD, GG) launch_mma<K, DD, GG>(v, q, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, max_ctas, n_ctas_out, after_write, ap, s)
 #define HS_MMA_G(K, DD) \
     switch (G) { \
         case 1: return HS_MMA_RUN(K, DD, 1); \

@@ -304,9 +304,8 @@ __device__ __forceinline__ void load_sincos8(const uint16_t *srow, const uint16_
     }
 }
 
-// Loads the 8 bf16 elements [d0, d0+8) of a row, rotated when sin != NULL.
-__device__ __forceinline__ void load_row8_rope(const uint16_t *row, int d0, const uint16_t *sin, const uint16_t *cos,
-                                               int pos, int rotary_dim, float (&x)[8]) {
+// The 8 bf16 elements [d0, d0+8) of a row, rotated when sin != NULL.
+__device__ __forceinline__ uint4 row8_rope(const uint16_t *row, int d0, const uint16_t *sin, const uint16_t *cos, int pos, int rotary_dim) {
     uint4 ow = *reinterpret_cast<const uint4 *>(row + d0);
     if (sin != nullptr && d0 < rotary_dim) {
         const int half = rotary_dim >> 1;
@@ -318,7 +317,11 @@ __device__ __forceinline__ void load_row8_rope(const uint16_t *row, int d0, cons
         ow.x = rope_pair(ow.x, pw.x, sw[0], cw[0], first); ow.y = rope_pair(ow.y, pw.y, sw[1], cw[1], first);
         ow.z = rope_pair(ow.z, pw.z, sw[2], cw[2], first); ow.w = rope_pair(ow.w, pw.w, sw[3], cw[3], first);
     }
-    unpack8_bf16(ow, x);
+    return ow;
+}
+__device__ __forceinline__ void load_row8_rope(const uint16_t *row, int d0, const uint16_t *sin, const uint16_t *cos,
+                                               int pos, int rotary_dim, float (&x)[8]) {
+    unpack8_bf16(row8_rope(row, d0, sin, cos, pos, rotary_dim), x);
 }
 
 }  // namespace hs

@@ -121,3 +121,55 @@ def test_pages_aligned_to_words(cuda, kind, d, g, shift):
         torch.cuda.synchronize()
     assert torch.equal(outs[0], outs[1])
     no_device_error()
+
+
+@pytest.mark.parametrize("hq,hkv,d,rotary", [(32, 8, 128, 128), (4, 2, 64, 64), (16, 2, 256, 64), (3, 3, 128, 0)])
+@pytest.mark.parametrize("page_tokens", [0, 40, 256])
+def test_bf16_step_writes_its_token(cuda, hq, hkv, d, rotary, page_tokens):
+    """decode_append without positions (the attention kernel writes the new token of every sequence) leaves the same cache and gives
+    the same output as the write kernel followed by the attention, bit for bit - also where the rotation table ends."""
+    from hyprstream_b200 import ffi, kv_cache as kc, ops
+
+    lens = [1, 2, 16, 17, 32, 40, 41, 639]
+    g = torch.Generator().manual_seed(d + page_tokens)
+    q = torch.randn(len(lens), hq, d, generator=g).bfloat16().to(cuda)
+    kn, vn = (torch.randn(len(lens), 1, hkv, d, generator=g).bfloat16().to(cuda) for _ in range(2))
+    old = [[torch.randn(1, l, hkv, d, generator=g).bfloat16().to(cuda) for _ in range(2)] for l in lens]
+    tables = (None, None) if not rotary else tuple(torch.randn(600, rotary // 2, generator=g).bfloat16().to(cuda) for _ in range(2))
+    sl = torch.tensor(lens, dtype=torch.int32, device=cuda)
+    results = []
+    for dst in (sl - 1, None):
+        pool = kc.BlockPool(sum((l + page_tokens - 1) // page_tokens for l in lens), hkv, d, cuda, kind=0, page_tokens=page_tokens) if page_tokens else None
+        caches = []
+        for i, kv in enumerate(old):
+            c = kc.LayerKVCache.new_paged(1 << 20, pool, owner=i) if pool else kc.LayerKVCache(1 << 20, kc.KVQuantType.NONE, hkv, d, cuda)
+            c.update(*kv, 0)
+            caches.append(c)
+        view, keep = kc.make_view(caches)
+        out = ops.decode_append(q, kn, vn, view, dst, sl, sin=tables[0], cos=tables[1], rotary_dim=rotary)
+        torch.cuda.synchronize()
+        err = ffi.take_device_error()
+        assert err == (ffi.DEVERR_KV_WRITE_RANGE if rotary else 0)  # position 638 is past the 600 rows of the table
+        results.append([out] + [t for c in caches for t in c.get()])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_bf16_step_without_room_is_recorded(cuda):
+    """A length of 0 and one past the view's pages: recorded, nothing written, the other sequences served."""
+    from hyprstream_b200 import ffi, kv_cache as kc, ops
+
+    kc0 = [kc.LayerKVCache(64, kc.KVQuantType.NONE, 2, 64, cuda) for _ in range(3)]
+    g = torch.Generator().manual_seed(1)
+    for c in kc0:
+        c.update(*(torch.randn(1, 64, 2, 64, generator=g).bfloat16().to(cuda) for _ in range(2)), 0)
+    before = [t.clone() for c in kc0 for t in c.get()]
+    view, keep = kc.make_view(kc0)
+    q = torch.randn(3, 4, 64, generator=g).bfloat16().to(cuda)
+    kn, vn = (torch.randn(3, 1, 2, 64, generator=g).bfloat16().to(cuda) for _ in range(2))
+    out = ops.decode_append(q, kn, vn, view, None, torch.tensor([0, 30, 65], dtype=torch.int32, device=cuda))
+    torch.cuda.synchronize()
+    assert ffi.take_device_error() == ffi.DEVERR_KV_WRITE_RANGE | ffi.DEVERR_DECODE_RANGE
+    after = [t for c in kc0 for t in c.get()]
+    assert torch.equal(after[0], before[0]) and torch.equal(after[4], before[4]) and torch.equal(after[5], before[5])
+    assert torch.equal(after[2][0, 29], kn[1, 0]) and torch.equal(after[3][0, 29], vn[1, 0])
+    assert (out[0] == 0).all() and torch.isfinite(out.float()).all()
