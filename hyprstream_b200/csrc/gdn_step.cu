@@ -33,6 +33,8 @@ gdn_step_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w, 
                 const float *__restrict__ dt_bias, const uint16_t *__restrict__ z, const float *__restrict__ norm_weight, float eps,
                 float *__restrict__ state, uint16_t *__restrict__ y, int nk, int nv, float q_scale) {
     constexpr int R = kGsD / kGsWarps;  // state rows per thread
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the block's next layer or its QK norm may start
+    EndOfGridWait order;
     __shared__ __align__(16) float s_qk[2][kGsD];                         // q, k (normalised)
     __shared__ __align__(16) float s_vv[2][kGsD];                         // v of the current value head (two buffers by head parity)
     __shared__ __align__(16) float s_pm[kGsWarps][kGsD], s_pr[kGsWarps][kGsD];
@@ -175,7 +177,7 @@ gdn_step_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w, 
 // `has_state` (zeros for a sequence's very first token) and shifted in place; `state` is updated in place.
 int32_t gdn_step_fused(const void *mixed_qkv, const void *conv_weight, void *conv_state, int32_t has_state, const void *a_in, const void *b_in,
                        const float *neg_a_exp, const float *dt_bias, const void *z, const float *norm_weight, float eps, float *state, void *y,
-                       int32_t n_seqs, int32_t n_k_heads, int32_t n_v_heads, int32_t kernel_size, hs_stream_t stream) {
+                       int32_t n_seqs, int32_t n_k_heads, int32_t n_v_heads, int32_t kernel_size, bool overlap, hs_stream_t stream) {
     if (kernel_size != 4 && kernel_size != 2) return fail(HS_ERR_UNSUPPORTED, "hs_gdn_layer_forward: conv kernel size %d (supported: 2, 4)", kernel_size);
     if (!aligned(mixed_qkv, 8) || !aligned(z, 16) || !aligned(y, 16) || !aligned(norm_weight, 16) || !aligned(state, 16))
         return fail(HS_ERR_ARG, "hs_gdn_layer_forward: mixed_qkv must be 8-byte, z, y, norm_weight and rec_state 16-byte aligned");
@@ -184,7 +186,7 @@ int32_t gdn_step_fused(const void *mixed_qkv, const void *conv_weight, void *con
     const float q_scale = 1.0f / sqrtf(static_cast<float>(kGsD));
     prof_begin(s);
 #define HS_GS(KS)                                                                                                                  \
-    gdn_step_kernel<KS><<<grid, kGsThreads, 0, s>>>(                                                                               \
+    launch_maybe_overlapped(gdn_step_kernel<KS>, grid, kGsThreads, s, overlap,                                                     \
         reinterpret_cast<const uint16_t *>(mixed_qkv), reinterpret_cast<const uint16_t *>(conv_weight),                            \
         reinterpret_cast<uint16_t *>(conv_state), has_state, reinterpret_cast<const uint16_t *>(a_in),                             \
         reinterpret_cast<const uint16_t *>(b_in), neg_a_exp, dt_bias, reinterpret_cast<const uint16_t *>(z), norm_weight, eps, state,  \

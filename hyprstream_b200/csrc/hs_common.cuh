@@ -37,7 +37,7 @@ int32_t gdn_conv_state_shift(const void *mixed_qkv, const void *state_in, void *
 // One decode step of a DeltaNet layer in one kernel (gdn_step.cu); conv_state is read (when has_state) and shifted in place.
 int32_t gdn_step_fused(const void *mixed_qkv, const void *conv_weight, void *conv_state, int32_t has_state, const void *a_in, const void *b_in,
                        const float *neg_a_exp, const float *dt_bias, const void *z, const float *norm_weight, float eps, float *state, void *y,
-                       int32_t n_seqs, int32_t n_k_heads, int32_t n_v_heads, int32_t kernel_size, hs_stream_t stream);
+                       int32_t n_seqs, int32_t n_k_heads, int32_t n_v_heads, int32_t kernel_size, bool overlap, hs_stream_t stream);
 // hs_attn_prefill_causal with the gate's strides given (elements between tokens / between heads); prefill.cu
 int32_t prefill_causal_impl(const void *q, const void *k, const void *v, void *out, const void *gate, int64_t gate_ts, int64_t gate_hs,
                             int32_t n_seqs, int32_t q_len, int32_t kv_len, int32_t n_q_heads, int32_t n_kv_heads, int32_t head_dim,
@@ -104,10 +104,39 @@ struct AppendArgs {
 };
 int32_t kv_write_at_end(const hs_kv_view *view, const void *k_new, const void *v_new, int32_t n_seqs, const int32_t *seq_lens, const void *sin,
                         const void *cos, int32_t rotary_dim, int32_t n_positions, hs_stream_t stream);
+// hs_qk_norm_rope / hs_kv_norm_rope_quantize_write that may overlap the kernel before them (see launch_maybe_overlapped)
+int32_t qk_norm_rope_impl(const void *x, int64_t token_stride, int64_t head_stride, void *out, void *gate_out, const float *norm_weight, float eps,
+                          int32_t weight_plus_one, const void *sin, const void *cos, const int32_t *positions, int32_t n_positions, int32_t rotary_dim,
+                          int64_t n_tokens, int32_t n_heads, int32_t head_dim, bool overlap, hs_stream_t stream);
+int32_t kv_norm_rope_write_impl(const hs_kv_view *view, const void *k_proj, const void *v_new, int32_t n_seqs, int32_t n_tokens, const int32_t *dst_pos,
+                                const float *k_norm_weight, float eps, int32_t weight_plus_one, const void *sin, const void *cos, int32_t rotary_dim,
+                                int32_t n_positions, void *k_out, bool overlap, hs_stream_t stream);
 // the host objects' forms, for one sequence: position / length by value instead of in device memory (quant.cu)
 int32_t kv_write_at(const hs_kv_view *view, const void *k_new, const void *v_new, int32_t n_tokens, int32_t start_pos, const void *sin, const void *cos,
                     int32_t rotary_dim, int32_t n_positions, hs_stream_t stream);
 int32_t kv_gather_len(const hs_kv_view *view, int32_t len, void *k_out, void *v_out, hs_stream_t stream);
+
+// ---- kernels of one entry point that do not depend on one another ----
+// Such a kernel may start while the one before it in the stream still runs (programmatic dependent launch: the earlier one
+// triggers at its start), which hides launch latency, ramp and tail of small grids.  Order is kept for everybody behind them: an
+// overlapped kernel's blocks wait for the kernel before it at their end (EndOfGridWait), so when the last of a chain is complete
+// all of them are.  The wait is a no-op in an ordinary launch.
+struct EndOfGridWait {
+    __device__ __forceinline__ ~EndOfGridWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+};
+template <typename... Params, typename... Args>
+static inline void launch_maybe_overlapped(void (*kern)(Params...), dim3 grid, int block, cudaStream_t s, bool overlap, Args... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);  // (a failure is reported by check_launch)
+}
 
 // ---- device helpers --------------------------------------------------------------------------
 __device__ __forceinline__ float bf16_bits_to_f32(uint16_t b) { return __uint_as_float(static_cast<uint32_t>(b) << 16); }

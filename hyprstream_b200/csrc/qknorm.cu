@@ -28,6 +28,8 @@ qk_norm_rope_kernel(const uint16_t *__restrict__ x, int64_t token_stride, int64_
                     const uint16_t *__restrict__ sin, const uint16_t *__restrict__ cos, const int32_t *__restrict__ positions,
                     int n_positions, int rotary_dim, int64_t n_tokens, int n_heads, int *__restrict__ err) {
     constexpr int D = LPR * 8;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the write of the same layer's keys may start
+    EndOfGridWait order;
     const int64_t row = (static_cast<int64_t>(blockIdx.x) * kNormThreads + threadIdx.x) / LPR;  // (token, head)
     const int l = threadIdx.x % LPR, d0 = l * 8;
     const bool live = row < n_tokens * n_heads;  // dead lanes still take part in the shuffles
@@ -99,12 +101,9 @@ qk_norm_rope_kernel(const uint16_t *__restrict__ x, int64_t token_stride, int64_
 
 using namespace hs;
 
-extern "C" {
-
-int32_t hs_qk_norm_rope(const void *x, int64_t token_stride, int64_t head_stride, void *out, void *gate_out,
-                        const float *norm_weight, float eps, int32_t weight_plus_one, const void *sin, const void *cos,
-                        const int32_t *positions, int32_t n_positions, int32_t rotary_dim, int64_t n_tokens, int32_t n_heads,
-                        int32_t head_dim, hs_stream_t stream) {
+int32_t hs::qk_norm_rope_impl(const void *x, int64_t token_stride, int64_t head_stride, void *out, void *gate_out, const float *norm_weight, float eps,
+                              int32_t weight_plus_one, const void *sin, const void *cos, const int32_t *positions, int32_t n_positions,
+                              int32_t rotary_dim, int64_t n_tokens, int32_t n_heads, int32_t head_dim, bool overlap, hs_stream_t stream) {
     if (int32_t st = check_device()) return st;
     if (n_tokens < 0 || n_heads <= 0) return fail(HS_ERR_ARG, "hs_qk_norm_rope: bad sizes");
     if (head_dim != 64 && head_dim != 128 && head_dim != 256) return fail(HS_ERR_UNSUPPORTED, "hs_qk_norm_rope: head_dim %d (supported: 64, 128, 256)", head_dim);
@@ -131,7 +130,7 @@ int32_t hs_qk_norm_rope(const void *x, int64_t token_stride, int64_t head_stride
     if (blocks > 0x7fffffffLL) return fail(HS_ERR_ARG, "hs_qk_norm_rope: too many rows");
     cudaStream_t s = as_stream(stream);
 #define HS_QKN(L)                                                                                                                   \
-    qk_norm_rope_kernel<L><<<static_cast<unsigned>(blocks), kNormThreads, 0, s>>>(                                                  \
+    launch_maybe_overlapped(qk_norm_rope_kernel<L>, dim3(static_cast<unsigned>(blocks)), kNormThreads, s, overlap,                  \
         reinterpret_cast<const uint16_t *>(x), token_stride, head_stride, reinterpret_cast<uint16_t *>(out),                        \
         reinterpret_cast<uint16_t *>(gate_out), norm_weight, eps, weight_plus_one, reinterpret_cast<const uint16_t *>(sin),         \
         reinterpret_cast<const uint16_t *>(cos), positions, n_positions, rotary_dim, n_tokens, n_heads, err)
@@ -140,6 +139,16 @@ int32_t hs_qk_norm_rope(const void *x, int64_t token_stride, int64_t head_stride
     prof_end(s);
 #undef HS_QKN
     return check_launch("hs_qk_norm_rope");
+}
+
+extern "C" {
+
+int32_t hs_qk_norm_rope(const void *x, int64_t token_stride, int64_t head_stride, void *out, void *gate_out,
+                        const float *norm_weight, float eps, int32_t weight_plus_one, const void *sin, const void *cos,
+                        const int32_t *positions, int32_t n_positions, int32_t rotary_dim, int64_t n_tokens, int32_t n_heads,
+                        int32_t head_dim, hs_stream_t stream) {
+    return qk_norm_rope_impl(x, token_stride, head_stride, out, gate_out, norm_weight, eps, weight_plus_one, sin, cos, positions, n_positions, rotary_dim,
+                             n_tokens, n_heads, head_dim, false, stream);
 }
 
 }  // extern "C"

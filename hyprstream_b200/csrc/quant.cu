@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
     // a decode launch that follows as a programmatic dependent may start now (it waits for this grid's completion before
     // it reads the cache); a no-op for every other successor
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    EndOfGridWait order;  // (it may itself run beside the QK norm of the same layer)
     __shared__ IndexTable<KIND> tab;
     tab.fill();
     __syncthreads();
@@ -565,7 +566,7 @@ int32_t hs_rope_apply(const void *x, void *out, const void *sin, const void *cos
 
 static int32_t kv_write_impl(const char *who, const hs_kv_view *view, const void *k_new, const void *v_new, int32_t n_seqs, int32_t n_tokens,
                              const int32_t *dst_pos, const void *sin, const void *cos, int32_t rotary_dim, int32_t n_positions, hs::KNormArgs kn,
-                             hs_stream_t stream) {
+                             hs_stream_t stream, bool overlap = false) {
     if (int32_t st = check_device()) return st;
     if (int32_t st = validate_view(view)) return st;
     if (n_seqs < 0 || n_tokens < 0) return fail(HS_ERR_ARG, "%s: negative sizes", who);
@@ -589,8 +590,8 @@ static int32_t kv_write_impl(const char *who, const hs_kv_view *view, const void
     if (!err) return fail(HS_ERR_DEVICE, "%s: device error word unavailable", who);
     const uint16_t *k = reinterpret_cast<const uint16_t *>(k_new), *v = reinterpret_cast<const uint16_t *>(v_new);
     const uint16_t *sn = reinterpret_cast<const uint16_t *>(sin), *cs = reinterpret_cast<const uint16_t *>(cos);
-#define HS_KV_WRITE_N(K, N) do { if (wide) kv_write_kernel<K, 16, N><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); \
-                                 else kv_write_kernel<K, 8, N><<<grid, kQThreads, 0, s>>>(d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); } while (0)
+#define HS_KV_WRITE_N(K, N) do { if (wide) launch_maybe_overlapped(kv_write_kernel<K, 16, N>, grid, kQThreads, s, overlap, d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); \
+                                 else launch_maybe_overlapped(kv_write_kernel<K, 8, N>, grid, kQThreads, s, overlap, d, k, v, n_seqs, n_tokens, dst_pos, sn, cs, rotary_dim, n_positions, err, kn); } while (0)
 #define HS_KV_WRITE(K) do { if (kn.weight != nullptr) HS_KV_WRITE_N(K, true); else HS_KV_WRITE_N(K, false); } while (0)
     switch (view->kind) {
         case HS_KV_BF16: HS_KV_WRITE(HS_KV_BF16); break;
@@ -626,14 +627,21 @@ int32_t hs::kv_write_at_end(const hs_kv_view *view, const void *k_new, const voi
                          hs::KNormArgs{nullptr, 0.0f, 0, nullptr, -1}, stream);
 }
 
+int32_t hs::kv_norm_rope_write_impl(const hs_kv_view *view, const void *k_proj, const void *v_new, int32_t n_seqs, int32_t n_tokens,
+                                    const int32_t *dst_pos, const float *k_norm_weight, float eps, int32_t weight_plus_one, const void *sin,
+                                    const void *cos, int32_t rotary_dim, int32_t n_positions, void *k_out, bool overlap, hs_stream_t stream) {
+    if (!k_norm_weight) return fail(HS_ERR_ARG, "hs_kv_norm_rope_quantize_write: NULL norm weight (use hs_kv_quantize_write)");
+    return kv_write_impl("hs_kv_norm_rope_quantize_write", view, k_proj, v_new, n_seqs, n_tokens, dst_pos, sin, cos, rotary_dim, n_positions,
+                         hs::KNormArgs{k_norm_weight, eps, weight_plus_one, reinterpret_cast<uint16_t *>(k_out), 0}, stream, overlap);
+}
+
 extern "C" {
 
 int32_t hs_kv_norm_rope_quantize_write(const hs_kv_view *view, const void *k_proj, const void *v_new, int32_t n_seqs, int32_t n_tokens,
                                        const int32_t *dst_pos, const float *k_norm_weight, float eps, int32_t weight_plus_one, const void *sin,
                                        const void *cos, int32_t rotary_dim, int32_t n_positions, void *k_out, hs_stream_t stream) {
-    if (!k_norm_weight) return fail(HS_ERR_ARG, "hs_kv_norm_rope_quantize_write: NULL norm weight (use hs_kv_quantize_write)");
-    return kv_write_impl("hs_kv_norm_rope_quantize_write", view, k_proj, v_new, n_seqs, n_tokens, dst_pos, sin, cos, rotary_dim, n_positions,
-                         hs::KNormArgs{k_norm_weight, eps, weight_plus_one, reinterpret_cast<uint16_t *>(k_out), 0}, stream);
+    return kv_norm_rope_write_impl(view, k_proj, v_new, n_seqs, n_tokens, dst_pos, k_norm_weight, eps, weight_plus_one, sin, cos, rotary_dim, n_positions,
+                                   k_out, false, stream);
 }
 
 static int32_t gather_launch(const hs_kv_view *view, const int32_t *seq_lens, int32_t n_seqs, int32_t out_tokens, void *k_out, void *v_out,

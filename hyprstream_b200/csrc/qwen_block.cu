@@ -10,6 +10,8 @@
 //
 // This file is host code: it chains the library's own entry points and only carves their intermediates out of the
 // caller's workspace.
+#include <vector>
+
 #include "hs_common.cuh"
 
 namespace hs {
@@ -32,6 +34,23 @@ static GdnScratch gdn_scratch(const hs_gdn_layer_params *p, int64_t n_seqs, int6
     s.total = off;
     return s;
 }
+
+// Address ranges that the kernels of a block read (or also write).
+struct Spans {
+    struct Span { uintptr_t b, e; bool written; };
+    std::vector<Span> v;
+    void add(const void *p, int64_t bytes, bool written) {
+        const uintptr_t b = reinterpret_cast<uintptr_t>(p);
+        v.push_back({b, b + static_cast<uintptr_t>(bytes > 0 ? bytes : 0), written});
+    }
+    // nothing from index `first` on touches what the ranges before it write, or writes what they touch
+    bool apart(size_t first) const {
+        for (size_t i = first; i < v.size(); ++i)
+            for (size_t j = 0; j < first; ++j)
+                if ((v[i].written || v[j].written) && v[i].b < v[j].e && v[j].b < v[i].e) return false;
+        return true;
+    }
+};
 
 static int32_t check_gdn_params(const hs_gdn_layer_params *p, const char *who) {
     if (!p) return fail(HS_ERR_ARG, "%s: NULL layer parameters", who);
@@ -61,9 +80,9 @@ int64_t hs_gdn_layer_workspace_bytes(const hs_gdn_layer_params *params, int32_t 
     return static_cast<int64_t>(gdn_scratch(params, n_seqs, n_tokens, nullptr).total);
 }
 
-int32_t hs_gdn_layer_forward(const hs_gdn_layer_params *params, const void *mixed_qkv, const void *z, const void *a_in, const void *b_in,
-                             void *conv_state, float *rec_state, int32_t has_state, int32_t n_seqs, int32_t n_tokens, void *y,
-                             void *workspace, int64_t workspace_bytes, hs_stream_t stream) {
+static int32_t gdn_layer_forward_impl(const hs_gdn_layer_params *params, const void *mixed_qkv, const void *z, const void *a_in, const void *b_in,
+                                      void *conv_state, float *rec_state, int32_t has_state, int32_t n_seqs, int32_t n_tokens, void *y,
+                                      void *workspace, int64_t workspace_bytes, bool overlap, hs_stream_t stream) {
     if (int32_t st = check_device()) return st;
     if (int32_t st = check_gdn_params(params, "hs_gdn_layer_forward")) return st;
     if (n_seqs < 0 || n_tokens < 0) return fail(HS_ERR_ARG, "hs_gdn_layer_forward: negative sizes");
@@ -81,7 +100,7 @@ int32_t hs_gdn_layer_forward(const hs_gdn_layer_params *params, const void *mixe
     if (n_tokens == 1 && n_seqs <= 65535) {
         // a decode step: conv (with the conv_state shift), gates, the recurrent rule and RMSNormGated in one kernel
         return gdn_step_fused(mixed_qkv, params->conv_weight, conv_state, has_state, a_in, b_in, params->neg_a_exp, params->dt_bias, z, params->norm_weight,
-                              params->norm_eps, rec_state, y, n_seqs, params->n_k_heads, params->n_v_heads, params->kernel_size, stream);
+                              params->norm_eps, rec_state, y, n_seqs, params->n_k_heads, params->n_v_heads, params->kernel_size, overlap, stream);
     }
     // conv1d + SiLU + split + L2 norm + gates (qwen3_5.rs:627-701).  For a prompt q, k, v go to the chunked rule as bf16: that kernel
     // rounds q and k to bf16 first thing and v is a bf16 value already, so the results are the same and half the bytes move.
@@ -104,6 +123,13 @@ int32_t hs_gdn_layer_forward(const hs_gdn_layer_params *params, const void *mixe
                            stream);
 }
 
+int32_t hs_gdn_layer_forward(const hs_gdn_layer_params *params, const void *mixed_qkv, const void *z, const void *a_in, const void *b_in,
+                             void *conv_state, float *rec_state, int32_t has_state, int32_t n_seqs, int32_t n_tokens, void *y,
+                             void *workspace, int64_t workspace_bytes, hs_stream_t stream) {
+    return gdn_layer_forward_impl(params, mixed_qkv, z, a_in, b_in, conv_state, rec_state, has_state, n_seqs, n_tokens, y, workspace, workspace_bytes, false,
+                                  stream);
+}
+
 int64_t hs_qwen_attn_layer_workspace_bytes(const hs_qwen_attn_params *params, int32_t n_seqs, int32_t n_tokens) {
     if (!params || n_seqs < 0 || n_tokens < 0) return HS_ERR_ARG;
     const size_t rows = static_cast<size_t>(n_seqs) * n_tokens;
@@ -112,9 +138,9 @@ int64_t hs_qwen_attn_layer_workspace_bytes(const hs_qwen_attn_params *params, in
     return static_cast<int64_t>(2 * qb + kb) + (dec > 0 ? static_cast<int64_t>(up256(static_cast<size_t>(dec))) : 0);
 }
 
-int32_t hs_qwen_attn_layer_forward(const hs_qwen_attn_params *params, const void *q_proj, const void *k_proj, const void *v_proj,
-                                   const hs_kv_view *view, const int32_t *positions, const int32_t *dst_pos, const int32_t *seq_lens, int32_t n_seqs,
-                                   int32_t n_tokens, void *out, void *workspace, int64_t workspace_bytes, hs_stream_t stream) {
+static int32_t attn_layer_forward_impl(const hs_qwen_attn_params *params, const void *q_proj, const void *k_proj, const void *v_proj,
+                                       const hs_kv_view *view, const int32_t *positions, const int32_t *dst_pos, const int32_t *seq_lens, int32_t n_seqs,
+                                       int32_t n_tokens, void *out, void *workspace, int64_t workspace_bytes, bool overlap, hs_stream_t stream) {
     if (int32_t st = check_device()) return st;
     if (int32_t st = check_attn_params(params, "hs_qwen_attn_layer_forward")) return st;
     if (int32_t st = validate_view(view)) return st;
@@ -135,20 +161,27 @@ int32_t hs_qwen_attn_layer_forward(const hs_qwen_attn_params *params, const void
     void *query = w, *gate = w + qb, *k_rot = w + 2 * qb, *dec_ws = w + 2 * qb + kb;
     // q_proj rows are [n_q_heads, 2 * head_dim]: query half | gate half (qwen3_5.rs:965-967); (1 + w) QK-norm, partial RoPE.
     // A decode step copies the gate halves out (its kernel wants them dense); a prompt's attention reads them in place.
-    if (int32_t st = hs_qk_norm_rope(q_proj, static_cast<int64_t>(hq) * 2 * d, 2 * d, query, n_tokens == 1 ? gate : nullptr, params->q_norm_weight, params->norm_eps, 1, params->sin,
-                                     params->cos, positions, params->n_positions, params->rotary_dim, rows, hq, d, stream))
+    if (int32_t st = qk_norm_rope_impl(q_proj, static_cast<int64_t>(hq) * 2 * d, 2 * d, query, n_tokens == 1 ? gate : nullptr, params->q_norm_weight, params->norm_eps, 1, params->sin,
+                                     params->cos, positions, params->n_positions, params->rotary_dim, rows, hq, d, overlap, stream))
         return st;
     // K: norm + rotation + cache update in one pass over the new keys (qwen3_5.rs:971-999); a prompt also keeps the normed,
     // rotated keys in bf16 for its own attention.  The keys' RoPE rows are their cache positions dst_pos[s] + t, which is
-    // what `positions` holds for the queries.
-    if (int32_t st = hs_kv_norm_rope_quantize_write(view, k_proj, v_proj, n_seqs, n_tokens, dst_pos, params->k_norm_weight, params->norm_eps, 1, params->sin,
-                                                    params->cos, params->rotary_dim, params->n_positions, n_tokens == 1 ? nullptr : k_rot, stream))
+    // what `positions` holds for the queries.  It needs nothing of the pass over q and may run beside it.
+    if (int32_t st = kv_norm_rope_write_impl(view, k_proj, v_proj, n_seqs, n_tokens, dst_pos, params->k_norm_weight, params->norm_eps, 1, params->sin,
+                                                    params->cos, params->rotary_dim, params->n_positions, n_tokens == 1 ? nullptr : k_rot, true, stream))
         return st;
     if (n_tokens == 1)
         return hs_attn_decode(query, view, seq_lens, n_seqs, hq, params->softmax_scale, out, gate, dec_ws,
                               hs_attn_decode_workspace_bytes(n_seqs, hq, d), nullptr, nullptr, stream);
     return hs::prefill_causal_impl(query, k_rot, v_proj, out, static_cast<const uint16_t *>(q_proj) + d, static_cast<int64_t>(hq) * 2 * d, 2 * d, n_seqs, n_tokens,
                                    n_tokens, hq, hkv, d, params->softmax_scale, stream);
+}
+
+int32_t hs_qwen_attn_layer_forward(const hs_qwen_attn_params *params, const void *q_proj, const void *k_proj, const void *v_proj,
+                                   const hs_kv_view *view, const int32_t *positions, const int32_t *dst_pos, const int32_t *seq_lens, int32_t n_seqs,
+                                   int32_t n_tokens, void *out, void *workspace, int64_t workspace_bytes, hs_stream_t stream) {
+    return attn_layer_forward_impl(params, q_proj, k_proj, v_proj, view, positions, dst_pos, seq_lens, n_seqs, n_tokens, out, workspace, workspace_bytes, false,
+                                   stream);
 }
 
 int64_t hs_qwen_block_workspace_bytes(const hs_gdn_layer_params *gdn, int32_t n_gdn, const hs_qwen_attn_params *attn, int32_t n_seqs,
@@ -172,15 +205,45 @@ int32_t hs_qwen_block_forward(const hs_gdn_layer_params *gdn, const hs_gdn_layer
                               int64_t workspace_bytes, hs_stream_t stream) {
     if (n_gdn < 0 || (n_gdn > 0 && (!gdn || !gdn_io))) return fail(HS_ERR_ARG, "hs_qwen_block_forward: bad DeltaNet layer arrays");
     if ((attn == nullptr) != (attn_io == nullptr)) return fail(HS_ERR_ARG, "hs_qwen_block_forward: attention parameters and inputs go together");
+    // A decode step's layers read only what the caller has handed in, so each kernel may start beside the one before it - unless
+    // buffers are shared between layers: every layer's inputs, states and outputs are compared with those of the layers before.
+    Spans spans;
     for (int i = 0; i < n_gdn; ++i) {
         const hs_gdn_layer_io &io = gdn_io[i];
-        if (int32_t st = hs_gdn_layer_forward(gdn + i, io.mixed_qkv, io.z, io.a_in, io.b_in, io.conv_state, io.rec_state, has_state, n_seqs, n_tokens, io.y,
-                                              workspace, workspace_bytes, stream))
+        bool overlap = false;
+        if (n_tokens == 1 && has_state && n_seqs > 0) {
+            const hs_gdn_layer_params &p = gdn[i];
+            const int64_t n = n_seqs, vd = static_cast<int64_t>(p.n_v_heads) * p.head_v_dim, conv = 2LL * p.n_k_heads * p.head_k_dim + vd;
+            const size_t first = spans.v.size();
+            spans.add(io.mixed_qkv, n * conv * 2, false);
+            spans.add(io.z, n * vd * 2, false);
+            spans.add(io.a_in, n * p.n_v_heads * 2, false);
+            spans.add(io.b_in, n * p.n_v_heads * 2, false);
+            spans.add(io.conv_state, n * conv * (p.kernel_size - 1) * 2, true);
+            spans.add(io.rec_state, n * vd * p.head_k_dim * 4, true);
+            spans.add(io.y, n * vd * 2, true);
+            overlap = i > 0 && spans.apart(first);
+        }
+        if (int32_t st = gdn_layer_forward_impl(gdn + i, io.mixed_qkv, io.z, io.a_in, io.b_in, io.conv_state, io.rec_state, has_state, n_seqs, n_tokens, io.y,
+                                                workspace, workspace_bytes, overlap, stream))
             return st;
     }
-    if (attn)
-        return hs_qwen_attn_layer_forward(attn, attn_io->q_proj, attn_io->k_proj, attn_io->v_proj, attn_io->view, attn_io->positions, attn_io->dst_pos,
-                                          attn_io->seq_lens, n_seqs, n_tokens, attn_io->out, workspace, workspace_bytes, stream);
+    if (attn) {
+        bool overlap = false;
+        if (n_tokens == 1 && has_state && n_seqs > 0 && n_gdn > 0) {
+            const int64_t n = n_seqs, d = attn->head_dim;
+            const size_t first = spans.v.size();
+            spans.add(attn_io->q_proj, n * attn->n_q_heads * 2 * d * 2, false);
+            spans.add(attn_io->k_proj, n * attn->n_kv_heads * d * 2, false);
+            spans.add(attn_io->v_proj, n * attn->n_kv_heads * d * 2, false);
+            spans.add(attn_io->positions, n * 4, false);
+            spans.add(attn_io->dst_pos, n * 4, false);
+            spans.add(workspace, workspace_bytes, true);
+            overlap = spans.apart(first);
+        }
+        return attn_layer_forward_impl(attn, attn_io->q_proj, attn_io->k_proj, attn_io->v_proj, attn_io->view, attn_io->positions, attn_io->dst_pos,
+                                       attn_io->seq_lens, n_seqs, n_tokens, attn_io->out, workspace, workspace_bytes, overlap, stream);
+    }
     return HS_OK;
 }
 
