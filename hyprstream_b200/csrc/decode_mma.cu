@@ -14,7 +14,9 @@
 //     MMA's 8 columns is free and carries lo (one MMA for both); with 8 heads lo takes an MMA and an accumulator of its own;
 //   * the warps of a CTA merge their sums at the end of a sequence and write one partial per (CTA, sequence).
 // Measured against the CUDA-core form (a cold launch by itself), bf16, 32 / 8 heads x 128: 16 paged sequences of 100 to 6,000 tokens
-// (247 MB) 150 -> 44.0 us = 5.6 TB/s; one sequence of 4,096 tokens 23.3 -> 9.3 us.
+// (247 MB) 150 -> 44.0 us = 5.6 TB/s; one sequence of 4,096 tokens 23.3 -> 9.3 us.  Whole steps of 32 sequences of 4,096 to 8,192
+// tokens: NF4 16 / 2 x 256 617 -> 121 us, NF4 32 / 8 x 64 321 -> 101, NF4 8 / 8 x 128 208 -> 158, int8 32 / 8 x 64 289 -> 97, int8
+// 8 / 8 x 128 251 -> 127 us (floors 16 to 65 us: the warps' instruction chain bounds the codes, not HBM).
 #include "hs_common.cuh"
 #include "quant_dev.cuh"
 

@@ -923,7 +923,7 @@ static int32_t launch_tc(const ViewDev &v, const uint16_t *q, const int32_t *seq
     using LT = TcLayout<FOURBIT, BPR, SF16, WIDE>;
     auto kern = decode_int8_tc_kernel<FOURBIT, BPR, SF16, WIDE>;
     // per instantiation and device: 0 = not configured, 1 / 2 = CTAs per SM of the cooperative grid, -1 = the device does not
-    // take this kernel as a cooperative launch (the generic kernel serves it)
+    // take this kernel as a cooperative launch (decode_mma.cu serves it)
     static PerDeviceState config;
     const int dev = current_device();
     int ctas_per_sm = config.get(dev);
@@ -977,14 +977,14 @@ static int32_t launch_tc(const ViewDev &v, const uint16_t *q, const int32_t *seq
         *fused_out = 1;
         return HS_OK;
     }
-    cudaGetLastError();  // refused (e.g. the device is shared and cannot hold the whole grid): the generic kernel takes over for good
+    cudaGetLastError();  // refused (e.g. the device is shared and cannot hold the whole grid): decode_mma.cu takes over for good
     config.set(dev, -1);
     return HS_OK;
 }
 
 // Returns HS_OK and sets *n_ctas_out (> 0) and *merged_out = 1 when the tensor-core kernel took the launch (it
 // merges its own partials, which needs a cooperative launch); *n_ctas_out = 0 when the shape is not covered or
-// the device refuses cooperative launches, and the caller should use the generic kernel.
+// the device refuses cooperative launches, and the caller should use decode_mma.cu.
 int32_t decode_int8_tc_try(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads,
                            float softmax_scale, float *o_part, float *lse_part, int *err, cudaStream_t s, int *n_ctas_out,
                            uint16_t *out, const uint16_t *gate, float *o_shard, float *lse_shard, int *merged_out,

