@@ -36,6 +36,7 @@
 #include <cuda.h>
 
 #include "hs_common.cuh"
+#include "prefill_tc5_steps.h"
 
 namespace hs {
 
@@ -141,7 +142,7 @@ __device__ __forceinline__ void t5_tma_load(uint32_t dst, const CUtensorMap *map
 }
 
 struct T5Bars {
-    uint64_t q, kfull[kT5Stages], vfull[kT5Stages], kempty[kT5Stages], vempty[kT5Stages], sfull[2][2], pready[2][2], odone[2];
+    uint64_t q, kfull[kT5Stages], vfull[kT5Stages], kempty[kT5Stages], vempty[kT5Stages], sfull[2][2], pready[2][2], odone[2][kT5OBars];
 };
 
 __device__ __forceinline__ uint32_t t5_pack_bf16x2(float lo, float hi) {
@@ -218,7 +219,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         for (int s = 0; s < kT5Stages; ++s) { init(&bars.kfull[s], 1); init(&bars.vfull[s], 1); init(&bars.kempty[s], users); init(&bars.vempty[s], users); }
         for (int i = 0; i < 2; ++i) {
             for (int k = 0; k < 2; ++k) { init(&bars.sfull[i][k], 1); init(&bars.pready[i][k], kT5M / 32); }
-            init(&bars.odone[i], 1);
+            for (int k = 0; k < kT5OBars; ++k) init(&bars.odone[i][k], 1);
         }
         s_abort = *reinterpret_cast<volatile uint32_t *>(err + 1) == launch_id ? 1 : 0;  // a time-out recorded by this launch ends its later CTAs at once
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -291,7 +292,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
                 for (int ks = 0; ks < kT5S / 16; ++ks)
                     t5_mma_ts(tO, tS + hf * kT5S + ks * 8, dv0 + ((2 * st * kTileBytes + hf * kStepBytes + ks * 2048) >> 4), idesc_pv, (u > 0 || ks > 0) ? 1u : 0u);
-                t5_commit(t5_s32(&bars.odone[x]));
+                t5_commit(t5_s32(&bars.odone[x][t5_odone_bar(hf)]));  // (u - hf is even)
                 if (hf == 1 || u == nx - 1) t5_commit(t5_s32(&bars.vempty[st]));
             }
             __syncwarp();
@@ -376,7 +377,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             } else {
                 const bool need = m_new - m_used > kT5RescaleThreshold;  // false while both are -inf (NaN compares false)
                 if (__any_sync(0xffffffffu, need)) {
-                    ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x]), (u - 1) & 1, abort_flag));
+                    ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x][t5_odone_bar(u - 1)]), t5_odone_parity(u - 1), abort_flag));
                     if (!ok) break;
                     t5_fence_after();
                     const float f = need ? exp2f(m_used - m_new) : 1.0f;
@@ -438,9 +439,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (lane == 0) t5_arrive(t5_s32(&bars.pready[x][u & 1]));
         }
         // ---- epilogue ----
-        // (the last scores prove P.V_{nt-3} complete, no more: the parity of step nt - 1 can be told only once step nt - 2 is in)
-        if (ok && nt > 1) ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x]), (nt - 2) & 1, abort_flag));
-        if (ok && nt > 0) ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x]), (nt - 1) & 1, abort_flag));
+        if (ok && nt > 0) ok = __all_sync(0xffffffffu, t5_wait(t5_s32(&bars.odone[x][t5_odone_bar(nt - 1)]), t5_odone_parity(nt - 1), abort_flag));
         if (ok && nt > 0) {
             t5_fence_after();
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
