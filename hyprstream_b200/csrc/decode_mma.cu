@@ -203,10 +203,10 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
             const unsigned char *k0 = reinterpret_cast<const unsigned char *>(kp[page0]), *v0 = reinterpret_cast<const unsigned char *>(vp[page0]);
             constexpr int kPer = kMmTile * kChunks / 32, kRows = 32 / kChunks;  // copies per lane and operand; rows the warp covers per copy
             const int row0 = lane / kChunks, c = lane % kChunks;
-            // The step's new token (bf16 caches; LayerKVCache::update in the same launch, kv_cache.rs:1275-1496): the warp that fetches a
-            // sequence's last tile takes the token's K (rotated) and V row of its kv head from the inputs, writes them to the cache -
-            // the bits the write kernel writes - and puts them into the ring in place of a copy.  A position past the rotation
-            // table is recorded and its K row left as it is, as the write kernel does.
+            // The step's new token (bf16 cache of one sequence, whose tokens nobody else looks at; LayerKVCache::update in the same
+            // launch, kv_cache.rs:1275-1496): the warp that fetches the last tile takes the token's K (rotated) and V row of its kv head
+            // from the inputs, writes them to the cache - the bits the write kernel writes - and puts them into the ring in place of
+            // a copy.  A position past the rotation table is recorded and its K row left as it is, as the write kernel does.
             int k_row = -1, v_row = -1;  // rows of this tile that do not come from the cache
             if constexpr (!kQuant) {
                 const int pos = f_len - 1;
@@ -575,7 +575,7 @@ static int32_t launch_mma(const ViewDev &v, const uint16_t *q, const int32_t *se
     return HS_OK;
 }
 
-// `ap` (bf16 caches only, else k_new == NULL): the step's new tokens.  *n_ctas_out = CTAs per kv head, *tile_out = tokens per tile, as the merge kernel needs them.
+// `ap` (a bf16 cache of one sequence in one page, else k_new == NULL): the step's new token.  *n_ctas_out = CTAs per kv head, *tile_out = tokens per tile, as the merge kernel needs them.
 int32_t decode_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
                    float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, const AppendArgs &ap, cudaStream_t s) {
     *tile_out = kMmTile;

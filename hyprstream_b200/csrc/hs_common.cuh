@@ -95,8 +95,9 @@ struct ShardArgs {
     long long rows_cap;
 };
 
-// One new token per sequence that the decode kernel writes into the cache itself (int8 caches) before it attends:
-// k_new == NULL: off.  The token of sequence s goes to position seq_lens[s] - 1.
+// One new token per sequence that the decode kernel writes into the cache itself before it attends (int8 caches on decode_tc.cu;
+// a bf16 cache of one sequence in one page on decode_mma.cu); k_new == NULL: off.  The token of sequence s goes to position
+// seq_lens[s] - 1.
 struct AppendArgs {
     const uint16_t *k_new, *v_new;  // bf16 [n_seqs, 1, n_kv_heads, head_dim]
     const uint16_t *sin, *cos;      // optional fused K rotation

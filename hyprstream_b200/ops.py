@@ -177,8 +177,8 @@ def decode_append(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, vie
                   rotary_dim: int = 0, gate: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
                   workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Cache update of one new token per sequence + decode attention as one call (hs_attn_decode_append; llama.rs:598-640): the
-    new token of sequence s goes to ``dst_pos[s]``, or with ``dst_pos=None`` to ``seq_lens[s] - 1`` - then, on an int8 cache, the
-    attention kernel writes it itself (one launch per step).
+    new token of sequence s goes to ``dst_pos[s]``, or with ``dst_pos=None`` to ``seq_lens[s] - 1`` - then the attention kernel may write it
+    itself: int8 caches of the two shapes of the cooperative kernel (rows that share pages give positions), a bf16 cache of one sequence.
     q bf16 [n_seqs, Hq, D]; k_new, v_new bf16 [n_seqs, 1, Hkv, D]; dst_pos, seq_lens int32 [n_seqs]."""
     _need_cuda(q, k_new, v_new, dst_pos, seq_lens, sin, cos, gate)
     n_seqs, hq, d = q.shape

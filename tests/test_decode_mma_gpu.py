@@ -173,3 +173,64 @@ def test_bf16_step_without_room_is_recorded(cuda):
     assert torch.equal(after[0], before[0]) and torch.equal(after[4], before[4]) and torch.equal(after[5], before[5])
     assert torch.equal(after[2][0, 29], kn[1, 0]) and torch.equal(after[3][0, 29], vn[1, 0])
     assert (out[0] == 0).all() and torch.isfinite(out.float()).all()
+
+
+@pytest.mark.parametrize("kind,hq,hkv,d", [(0, 32, 8, 128), (0, 4, 2, 64), (0, 16, 2, 256), (1, 8, 2, 64), (2, 32, 8, 128)])
+@pytest.mark.parametrize("rows", [1, 2, 9])
+@pytest.mark.parametrize("positions", [False, True])
+def test_append_over_shared_pages(cuda, kind, hq, hkv, d, rows, positions):
+    """New tokens of one sequence handed in as rows (lengths L, L + 1, ... over the same pages): every token is in the cache before any
+    row attends, as with the write and the attention called one after the other.  rows = 1: a table that lists the new token's page twice."""
+    from hyprstream_b200 import ffi, ops
+
+    page, old, pps = 64, 210, 4
+    g = torch.Generator().manual_seed(d + rows)
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(cuda)  # noqa: E731
+    k, v, q = rnd(1, old, hkv, d), rnd(1, old, hkv, d), rnd(rows, hq, d)
+    kn, vn = rnd(rows, 1, hkv, d), rnd(rows, 1, hkv, d)
+    lens = torch.arange(old + 1, old + 1 + rows, dtype=torch.int32, device=cuda)
+    results = []
+    for append in (False, True):
+        row = {0: 2 * d, 1: d}.get(kind, d // 2) * hkv
+        bufs = [torch.zeros(pps, page * row, dtype=torch.uint8, device=cuda) for _ in range(2)]
+        bufs += [torch.zeros(pps, page * hkv * (d // 64), device=cuda) for _ in range(2 if kind else 0)]
+        tabs = [torch.tensor([[t[i].data_ptr() for i in range(pps)]] * rows, dtype=torch.int64, device=cuda) for t in bufs]
+        view = ffi.KVView(kind, ffi.SCALE_F32, 64, hkv, d, page, pps, 0, *[t.data_ptr() for t in tabs], *[None] * (4 - len(tabs)))
+        ops.kv_quantize_write(view, k, v, torch.zeros(1, dtype=torch.int32, device=cuda))
+        if rows == 1:
+            for t in tabs:
+                t[0, 0] = t[0, old // page]
+        if append:
+            out = ops.decode_append(q, kn, vn, view, lens - 1 if positions else None, lens)
+        else:
+            ops.kv_quantize_write(view, kn, vn, lens - 1)
+            out = ops.decode_attention(q, view, lens)
+        results.append([out] + bufs)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    no_device_error()
+
+
+@pytest.mark.parametrize("hq,hkv,d,rotary", [(32, 8, 128, 128), (4, 2, 64, 64), (16, 2, 256, 64), (3, 3, 128, 0)])
+@pytest.mark.parametrize("length", [1, 2, 16, 17, 32, 63, 64, 639])
+def test_bf16_step_of_one_sequence_writes_its_token(cuda, hq, hkv, d, rotary, length):
+    """One sequence in one page: the attention kernel writes the token, and cache and output are those of the two kernels, bit for bit -
+    also where the rotation table ends."""
+    from hyprstream_b200 import ffi, kv_cache as kc, ops
+
+    g = torch.Generator().manual_seed(d + length)
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(cuda)  # noqa: E731
+    q, kn, vn, old = rnd(1, hq, d), rnd(1, 1, hkv, d), rnd(1, 1, hkv, d), [rnd(1, length, hkv, d) for _ in range(2)]
+    tables = (None, None) if not rotary else (rnd(600, rotary // 2), rnd(600, rotary // 2))
+    sl = torch.tensor([length], dtype=torch.int32, device=cuda)
+    results = []
+    for dst in (sl - 1, None):
+        c = kc.LayerKVCache(1 << 20, kc.KVQuantType.NONE, hkv, d, cuda)
+        c.update(*old, 0)
+        view, keep = kc.make_view([c])
+        n0 = ffi.launch_count()
+        out = ops.decode_append(q, kn, vn, view, dst, sl, sin=tables[0], cos=tables[1], rotary_dim=rotary)
+        assert ffi.launch_count() - n0 == (2 if dst is None else 3)
+        torch.cuda.synchronize()
+        assert ffi.take_device_error() == (ffi.DEVERR_KV_WRITE_RANGE if rotary and length > 600 else 0)
+        results.append([out, *c.get()])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
