@@ -114,6 +114,7 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
     extern __shared__ __align__(128) unsigned char mm_smem[];
     // the merge kernel that follows as a programmatic dependent may start; it waits for this grid before it reads anything
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    EndOfGridWait order;  // (also blocks without work: the merge waits for this grid alone, and the write in front of it may still run)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kvh = blockIdx.y, H = view.n_kv_heads;
     const int64_t cta = blockIdx.x;

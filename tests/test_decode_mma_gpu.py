@@ -234,3 +234,29 @@ def test_bf16_step_of_one_sequence_writes_its_token(cuda, hq, hkv, d, rotary, le
         assert ffi.take_device_error() == (ffi.DEVERR_KV_WRITE_RANGE if rotary and length > 600 else 0)
         results.append([out, *c.get()])
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("kind,hq,hkv,d", [(0, 8, 2, 128), (1, 8, 2, 64), (2, 32, 8, 64), (1, 32, 8, 128)])
+def test_append_with_nothing_to_attend(cuda, kind, hq, hkv, d):
+    """Positions given and every length 0: no block of the attention has work, and still what follows on the stream sees the tokens that
+    the write kernel in front of it stores."""
+    from hyprstream_b200 import kv_cache as kc, ops
+
+    n = 64
+    g = torch.Generator().manual_seed(d)
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(cuda)  # noqa: E731
+    kn, vn, q = rnd(n, 1, hkv, d), rnd(n, 1, hkv, d), rnd(n, hq, d)
+    dst = torch.arange(n, dtype=torch.int32, device=cuda)
+    caches = [[kc.LayerKVCache(64, kc.KVQuantType(kind), hkv, d, cuda) for _ in range(n)] for _ in range(2)]
+    for c in caches[0] + caches[1]:
+        c._ensure_capacity(64)
+    (want, keep0), (got, keep1) = (kc.make_view(c) for c in caches)
+    full = torch.full((n,), 64, dtype=torch.int32, device=cuda)
+    ops.kv_quantize_write(want, kn, vn, dst)
+    ref = ops.kv_gather_dequantize(want, full, 64)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        out = ops.decode_append(q, kn, vn, got, dst, torch.zeros(n, dtype=torch.int32, device=cuda))
+        seen = ops.kv_gather_dequantize(got, full, 64)
+        assert (out == 0).all() and all(torch.equal(a, b) for a, b in zip(ref, seen))
+    no_device_error()
