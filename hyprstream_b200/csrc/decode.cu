@@ -29,13 +29,30 @@ decode_merge_kernel(const int32_t *__restrict__ seq_lens, int n_seqs, int n_q_he
                     const uint16_t *__restrict__ gate, float *__restrict__ o_shard, float *__restrict__ lse_shard) {
     __shared__ float4 s_num[kMergeThreads];
     const int r = blockIdx.x / n_q_heads, h = blockIdx.x - r * n_q_heads, lane = threadIdx.x & 31;
-    // every warp computes the tile prefix redundantly, one coalesced load per 32 sequences
+    // Tiles of all sequences, and of those in front of r, one coalesced load per 32 lengths.  A short list is summed by every warp for
+    // itself, a long one (there are n_seqs * n_q_heads CTAs) by all warps together.  bf16 32 / 8 heads x 128, up to 64 tokens, the whole
+    // call: 257 sequences 67.6 us together (256 by every warp: 85.4), 4,000 sequences 6,527 by every warp, 1,672 together.
     int64_t total = 0, before = 0;
-    for (int base = 0; base < n_seqs; base += 32) {
+    const bool together = n_seqs > 64;  // (one or two loads by every warp cost less than the barrier)
+    for (int base = together ? threadIdx.x & ~31 : 0; base < n_seqs; base += together ? kMergeThreads : 32) {
         const int i = base + lane;
         const unsigned t = i < n_seqs ? ceil_div_i(min(max(seq_lens[i], 0), cap), tile) : 0;
         total += __reduce_add_sync(0xffffffffu, t);
         before += __reduce_add_sync(0xffffffffu, i < r ? t : 0u);
+    }
+    if (together) {
+        __shared__ int64_t s_sum[2][kMergeThreads / 32];
+        if (lane == 0) {
+            s_sum[0][threadIdx.x >> 5] = total;
+            s_sum[1][threadIdx.x >> 5] = before;
+        }
+        __syncthreads();
+        total = before = 0;
+#pragma unroll
+        for (int w = 0; w < kMergeThreads / 32; ++w) {
+            total += s_sum[0][w];
+            before += s_sum[1][w];
+        }
     }
     const int64_t nt = ceil_div_i(min(max(seq_lens[r], 0), cap), tile);
     if (total < n_ctas) n_ctas = total > 0 ? static_cast<int>(total) : 1;  // the decode kernels never use more CTAs than tiles

@@ -260,3 +260,23 @@ def test_append_with_nothing_to_attend(cuda, kind, hq, hkv, d):
         seen = ops.kv_gather_dequantize(got, full, 64)
         assert (out == 0).all() and all(torch.equal(a, b) for a, b in zip(ref, seen))
     no_device_error()
+
+
+@pytest.mark.parametrize("n", [64, 65, 256, 257, 1025])
+def test_many_short_sequences(cuda, n):
+    """Batches whose lengths the merge sums warp by warp (up to 64) and block-wide (more), sequences of no tokens among them."""
+    from hyprstream_b200 import ffi, ops
+
+    hq, hkv, d, page = 4, 2, 64, 48
+    g = torch.Generator(device=cuda).manual_seed(n)
+    k, v = (torch.randn(n, page, hkv, d, device=cuda, generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(n, hq, d, device=cuda, generator=g).bfloat16()
+    lens = torch.randint(0, page + 1, (n,), dtype=torch.int32, device=cuda, generator=g)
+    tabs = [t.data_ptr() + torch.arange(n, device=cuda) * (page * hkv * d * 2) for t in (k, v)]
+    out = ops.decode_attention(q, ffi.KVView(0, 0, 64, hkv, d, page, 1, 0, *[t.data_ptr() for t in tabs], None, None), lens)
+    kk, vv = (t.double().repeat_interleave(hq // hkv, 2) for t in (k, v))
+    s = torch.einsum("nhd,nlhd->nhl", q.double(), kk) / math.sqrt(d)
+    s.masked_fill_(torch.arange(page, device=cuda) >= lens[:, None, None], -math.inf)
+    ref = torch.einsum("nhl,nlhd->nhd", s.softmax(-1).nan_to_num(0.0), vv)  # (no tokens: zeros)
+    assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 5e-4).all()  # as test_bf16_decode_every_shape
+    no_device_error()
