@@ -93,6 +93,13 @@ __device__ __forceinline__ void codes4_bf16(uint32_t w, uint32_t &lo, uint32_t &
     lo = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
     hi = __byte_perm(__float_as_uint(f[2]), __float_as_uint(f[3]), 0x7632);
 }
+// the next bf16 term of a table value: `rest` = what the terms before it leave.  Where they leave nothing of a value other than zero, the
+// smallest number of its sign: a block scale may be infinite, and infinity x 0 would spoil the value's own infinity (as a term of
+// a finite sum it is 2^-126 of the scale)
+__device__ __forceinline__ float next_term(float rest, float value) {
+    const float t = bf16_round(rest);
+    return t == 0.0f && value != 0.0f ? copysignf(1.17549435e-38f, value) : t;
+}
 // the values of code byte `k` (0..3) of w, high nibble first, as two bf16 pairs: upper terms in .x, lower terms (the rest, rounded to
 // bf16) in .y; `lut` = address of this lane's column, entries `stride` bytes apart
 template <int STRIDE>
@@ -161,7 +168,7 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
         const float *book = view.kind == HS_KV_NF4 ? c_nf4 : c_fp4;
         for (int e = warp * 64 + (lane & 1); e < warp * 64 + 64; e += 2) {  // a warp's quarter of the bytes, two at a time, 16 lanes a byte
             const float v0 = book[e >> 4], v1 = book[e & 15], u0 = bf16_round(v0), u1 = bf16_round(v1);
-            if ((lane >> 1) < LT::kLutCols) tab[e * LT::kLutCols + (lane >> 1)] = make_uint2(pack_bf16(u0, u1), pack_bf16(v0 - u0, v1 - u1));
+            if ((lane >> 1) < LT::kLutCols) tab[e * LT::kLutCols + (lane >> 1)] = make_uint2(pack_bf16(u0, u1), pack_bf16(next_term(v0 - u0, v0), next_term(v1 - u1, v1)));
         }
         lut = static_cast<uint32_t>(__cvta_generic_to_shared(tab)) + 8u * (lane & (LT::kLutCols - 1));
         __syncthreads();

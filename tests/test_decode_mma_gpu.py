@@ -280,3 +280,17 @@ def test_many_short_sequences(cuda, n):
     ref = torch.einsum("nhl,nlhd->nhd", s.softmax(-1).nan_to_num(0.0), vv)  # (no tokens: zeros)
     assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 5e-4).all()  # as test_bf16_decode_every_shape
     no_device_error()
+
+
+@pytest.mark.parametrize("d,g", [(64, 2), (128, 1), (128, 8), (256, 4)])
+def test_nf4_decode_infinite_value(cuda, d, g):
+    """An infinite V element makes its block's scale infinite and its own code the one of -1: the output of its column is an infinity, the rest
+    of the block (0 x infinity) NaN, and nothing else is touched."""
+    def edit(k, v):
+        v[0, 3, 0, 5] = math.inf
+        v[0, 4, 1, d - 1] = -math.inf
+    q, kvs, out = _run(cuda, 2 * g, 2, d, [20], 0, seed=4, edit=edit, kind=2)
+    o = out[0].float().view(2, g, d)
+    assert (o[0, :, 5] == -math.inf).all() and (o[1, :, d - 1] == -math.inf).all()
+    assert o[0, :, :64].isnan().sum().item() == o[1, :, d - 64:].isnan().sum().item() == 63 * g
+    assert torch.isfinite(o).sum().item() == o.numel() - 2 * 64 * g
