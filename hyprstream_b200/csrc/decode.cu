@@ -150,7 +150,7 @@ int32_t decode_int8_tc_try(const ViewDev &v, const uint16_t *q, const int32_t *s
 
 // decode_mma.cu: tensor-core kernel for every kind, head_dim and query group
 int32_t decode_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
-                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, const AppendArgs &ap, cudaStream_t s);
+                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, bool exact, const AppendArgs &ap, cudaStream_t s);
 
 // ---- decode scratch that lives inside the library ------------------------------------------------
 // Backing store of hs_attn_decode_static(): the split-KV partials go here instead of into a workspace the
@@ -258,7 +258,8 @@ int32_t hs::decode_impl(const void *q, const hs_kv_view *view, const int32_t *se
                                         "all-gather and hs_attn_merge_partials_strided for this shape");
     }
     if (st == HS_OK && tc_ctas == 0) {
-        st = decode_mma(v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, decode_max_ctas(), &n_ctas, &tile, after_write != 0, append ? *append : AppendArgs{}, s);
+        st = decode_mma(v, qp, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, decode_max_ctas(), &n_ctas, &tile, after_write != 0, o_shard != nullptr,
+                        append ? *append : AppendArgs{}, s);
     }
     prof_end(s);
     if (st != HS_OK) return st;

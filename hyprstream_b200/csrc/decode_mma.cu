@@ -11,7 +11,12 @@
 //     integers code - 127, 4-bit codes as two bf16 terms of the table values
 //     (one lookup per code byte; V's nibbles of two neighbouring tokens are mixed into bytes first);
 //   * P (times V's block scale) keeps 16 bits of mantissa: p = hi + lo, both bf16.  With up to 4 query heads the second half of the
-//     MMA's 8 columns is free and carries lo (one MMA for both); with 8 heads lo takes an MMA and an accumulator of its own;
+//     MMA's 8 columns is free and carries lo (one MMA for both); with 8 heads lo takes an MMA and an accumulator of its own.  A bf16
+//     output is as near to 64 bits as with fp32 P (1.4e-3 to 1.8e-3: its own rounding).  fp32 results are not (1.6e-6 to 4.6e-6 in
+//     place of 3e-7), so a caller who takes them (EXACT: a shard's output and log-sum-exp) gets a third term of P and of the NF4
+//     values, all their products above 2^-24, and a tile's sum added to the accumulator by fp32 additions: 2.3e-7 to 3.9e-7.  32
+//     sequences of 4,096 to 8,192 tokens, EXACT against two terms (and the CUDA-core form): bf16 32 / 8 x 128 140 / 136 (416) us, int8
+//     8 / 8 x 128 125 / 119 (240), NF4 16 / 2 x 256 171 / 117 (555), NF4 8 / 8 x 128 230 / 152 (172: the third lookup);
 //   * the warps of a CTA merge their sums at the end of a sequence and write one partial per (CTA, sequence).
 // Measured against the CUDA-core form (a cold launch by itself), bf16, 32 / 8 heads x 128: 16 paged sequences of 100 to 6,000 tokens
 // (247 MB) 150 -> 44.0 us = 5.6 TB/s; one sequence of 4,096 tokens 23.3 -> 9.3 us.  Whole steps of 32 sequences of 4,096 to 8,192
@@ -27,7 +32,7 @@ constexpr int kMmThreads = kMmWarps * 32;
 constexpr int kMmTile = 16;  // tokens per tile of the flat partition = one warp step
 
 // KIND: HS_KV_BF16, HS_KV_INT8, or HS_KV_NF4 for both 4-bit kinds (the table is chosen at run time).
-template <int KIND, int D, int G>
+template <int KIND, int D, int G, bool EXACT>
 struct MmLayout {
     static constexpr bool kQuant = KIND != HS_KV_BF16;
     static constexpr int kRow = KIND == HS_KV_BF16 ? D * 2 : (KIND == HS_KV_INT8 ? D : D / 2);  // bytes of one (token, head) row
@@ -41,10 +46,13 @@ struct MmLayout {
     static constexpr int kMergeOff = kMmWarps * kStages * kTileBytes;
     static constexpr int kMlOff = kMergeOff + kMmWarps * G * kORow * 4;
     // 4-bit kinds: uint2 [256][kLutCols], code byte -> both values as bf16 pairs (upper terms, lower terms).  8 columns, two
-    // lanes of a half warp each (16 would be free of bank conflicts and cost a CTA per SM)
+    // lanes of a half warp each (16 would be free of bank conflicts and cost a CTA per SM).  FP4 needs the upper terms only; the rule
+    // does not tell it from NF4 (8 / 8 x 128, 32 sequences of 4,096 to 8,192 tokens: 150 us, the CUDA-core form 173)
     static constexpr int kLutCols = 8;
     static constexpr int kLutOff = (kMlOff + kMmWarps * G * 2 * 4 + 127) / 128 * 128;
-    static constexpr int kTotal = kLutOff + (kQuant && KIND != HS_KV_INT8 ? 256 * kLutCols * 8 : 0);
+    static constexpr int kLut2Cols = 8;  // EXACT: uint32_t [256][kLut2Cols], the pairs' third terms
+    static constexpr int kLut2Off = kLutOff + (kQuant && KIND != HS_KV_INT8 ? 256 * kLutCols * 8 : 0);
+    static constexpr int kTotal = kLut2Off + (EXACT && kQuant && KIND != HS_KV_INT8 ? 256 * kLut2Cols * 4 : 0);
     // codes take several times the instructions per byte that bf16 rows take: as many warps as the registers allow (a warp's chain
     // of lookups, MMAs and shuffles is latency, not throughput)
     static constexpr int kWant = !kQuant || D == 256 || G == 8 ? 2 : (D == 128 ? 3 : 4);
@@ -110,11 +118,19 @@ __device__ __forceinline__ uint2 lut_pairs(uint32_t lut, uint32_t w, uint32_t k)
     return v;
 }
 
-template <int KIND, int D, int G>
-__global__ void __launch_bounds__(kMmThreads, MmLayout<KIND, D, G>::kCtasPerSm)
+template <int STRIDE>
+__device__ __forceinline__ uint32_t lut_third(uint32_t lut2, uint32_t w, uint32_t k) {
+    const uint32_t byte = __byte_perm(w, 0u, 0x4440u | k);
+    uint32_t v;
+    asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(byte * STRIDE + lut2));
+    return v;
+}
+
+template <int KIND, int D, int G, bool EXACT>
+__global__ void __launch_bounds__(kMmThreads, MmLayout<KIND, D, G, EXACT>::kCtasPerSm)
 decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *__restrict__ seq_lens, int n_seqs, int n_q_heads,
                   float scale_log2, float *__restrict__ o_part, float *__restrict__ lse_part, int *__restrict__ err, AppendArgs ap) {
-    using LT = MmLayout<KIND, D, G>;
+    using LT = MmLayout<KIND, D, G, EXACT>;
     constexpr bool kQuant = LT::kQuant, kFour = kQuant && KIND != HS_KV_INT8;
     constexpr int kChunks = LT::kChunks;           // 16-byte chunks of a row
     constexpr int kStages = LT::kStages;
@@ -160,8 +176,8 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
         if (at > 0) before_first += __shfl_sync(0xffffffffu, inc, at - 1);
         done = past != 0;
     }
-    constexpr uint32_t kLutStride = LT::kLutCols * 8;
-    uint32_t lut = 0;
+    constexpr uint32_t kLutStride = LT::kLutCols * 8, kLut2Stride = LT::kLut2Cols * 4;
+    uint32_t lut = 0, lut2 = 0;
     const bool two_terms = view.kind == HS_KV_NF4;  // (FP4 values are exact in bf16)
     if constexpr (kFour) {
         uint2 *tab = reinterpret_cast<uint2 *>(mm_smem + LT::kLutOff);
@@ -169,7 +185,13 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
         for (int e = warp * 64 + (lane & 1); e < warp * 64 + 64; e += 2) {  // a warp's quarter of the bytes, two at a time, 16 lanes a byte
             const float v0 = book[e >> 4], v1 = book[e & 15], u0 = bf16_round(v0), u1 = bf16_round(v1);
             if ((lane >> 1) < LT::kLutCols) tab[e * LT::kLutCols + (lane >> 1)] = make_uint2(pack_bf16(u0, u1), pack_bf16(next_term(v0 - u0, v0), next_term(v1 - u1, v1)));
+            if constexpr (EXACT) {
+                if ((lane >> 1) < LT::kLut2Cols)
+                    reinterpret_cast<uint32_t *>(mm_smem + LT::kLut2Off)[e * LT::kLut2Cols + (lane >> 1)] =
+                        pack_bf16(next_term(v0 - u0 - bf16_round(v0 - u0), v0), next_term(v1 - u1 - bf16_round(v1 - u1), v1));
+            }
         }
+        lut2 = static_cast<uint32_t>(__cvta_generic_to_shared(mm_smem + LT::kLut2Off)) + 4u * (lane & (LT::kLut2Cols - 1));
         lut = static_cast<uint32_t>(__cvta_generic_to_shared(tab)) + 8u * (lane & (LT::kLutCols - 1));
         __syncthreads();
     }
@@ -379,6 +401,11 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
                                 const uint2 v0 = lut_pairs<kLutStride>(lut, w, 2 * (s & 1)), v1 = lut_pairs<kLutStride>(lut, w, 2 * (s & 1) + 1);
                                 mma_bf16(s0, qa[4 * b + s][0], 0u, qa[4 * b + s][1], 0u, v0.x, v1.x);
                                 if (two_terms) mma_bf16(s1, qa[4 * b + s][0], 0u, qa[4 * b + s][1], 0u, v0.y, v1.y);
+                                if constexpr (EXACT) {
+                                    if (two_terms)
+                                        mma_bf16(s1, qa[4 * b + s][0], 0u, qa[4 * b + s][1], 0u, lut_third<kLut2Stride>(lut2, w, 2 * (s & 1)),
+                                                 lut_third<kLut2Stride>(lut2, w, 2 * (s & 1) + 1));
+                                }
                             }
                         }
                         const float2 ks = *reinterpret_cast<const float2 *>(sc + (b >> (kLog2(D / 64) - bpr_shift)) * kMmTile + nt * 8 + 2 * j);
@@ -416,19 +443,66 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
                     for (int i = 0; i < kLo; ++i) { Olo[i][0] *= c0; Olo[i][1] *= c1; Olo[i][2] *= c0; Olo[i][3] *= c1; }
                 }
             }
-            // P (times V's scale of a block) as two bf16 terms; ph / pl: the B operands of the upper and lower term
-            uint32_t ph[2], pl[2];
+            // P (times V's scale of a block) as two bf16 terms; ph / pl: the B operands of the upper and lower term.  EXACT: three terms,
+            // in 8 columns as far as they go: up to 2 heads, ph has them all; 4 heads, the third has an MMA of its own with pt, whose
+            // upper columns must carry something of P too (an infinite value times zero would be NaN): half of the upper term in
+            // this MMA and half in the first one's ph2; 8 heads, an MMA each.
+            uint32_t ph[2], pl[2], pt[2], ph2[2];
             auto split_p = [&](float2 v0, float2 v1) {
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
                     const float a = p[nt][0] * (nt ? v1.x : v0.x), b = p[nt][1] * (nt ? v1.y : v0.y);
+                    if constexpr (EXACT) {
+                        const uint32_t half = pack_bf16(0.5f * a, 0.5f * b);
+                        ph[nt] = pack_bf16(2.0f * bf16lo(half), 2.0f * bf16hi(half));
+                        const float ra = a - bf16lo(ph[nt]), rb = b - bf16hi(ph[nt]);
+                        pl[nt] = pack_bf16(ra, rb);
+                        pt[nt] = pack_bf16(ra - bf16lo(pl[nt]), rb - bf16hi(pl[nt]));
+                        if constexpr (G <= 2) {
+                            ph[nt] = g < G ? ph[nt] : (g / G == 2 ? pt[nt] : pl[nt]);
+                        } else if constexpr (G == 4) {
+                            ph2[nt] = low_half ? pl[nt] : half;
+                            pt[nt] = low_half ? pt[nt] : half;
+                            if (low_half) ph[nt] = pl[nt];
+                        }
+                        continue;
+                    }
                     ph[nt] = pack_bf16(a, b);
                     pl[nt] = pack_bf16(a - bf16lo(ph[nt]), b - bf16hi(ph[nt]));
                     if (low_half) ph[nt] = pl[nt];
                 }
             };
+            // EXACT: O^T += (all terms of A).P^T, the tile's sum on its own first: an MMA cuts its sum off at the accumulator's last
+            // bit, which over thousands of tokens is more than the rounding of as many additions
+            auto pv_exact = [&](int mt, const uint4 *a, int terms) {
+                float t[4] = {0.0f, 0.0f, 0.0f, 0.0f}, tl[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int i = 2; i >= 0; --i) {
+                    if (i >= terms) continue;
+                    if constexpr (G == 8) {
+                        if (i == 0) mma_bf16(tl, a[i].x, a[i].y, a[i].z, a[i].w, pt[0], pt[1]);
+                        if (i <= 1) mma_bf16(tl, a[i].x, a[i].y, a[i].z, a[i].w, pl[0], pl[1]);
+                    }
+                    if (G == 4 && i == 0) {
+                        mma_bf16(t, a[i].x, a[i].y, a[i].z, a[i].w, pt[0], pt[1]);
+                        mma_bf16(t, a[i].x, a[i].y, a[i].z, a[i].w, ph2[0], ph2[1]);
+                    } else {
+                        mma_bf16(t, a[i].x, a[i].y, a[i].z, a[i].w, ph[0], ph[1]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    O[mt][i] += t[i];
+                    if constexpr (G == 8) Olo[mt][i] += tl[i];
+                }
+            };
             // O^T += A.P^T; low: A is the lower term of the values
             auto pv = [&](int mt, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, bool low) {
+                if constexpr (EXACT) {
+                    const uint4 a = make_uint4(a0, a1, a2, a3);
+                    pv_exact(mt, &a, 1);
+                    return;
+                }
                 mma_bf16(O[mt], a0, a1, a2, a3, ph[0], ph[1]);
                 if constexpr (G == 8) {
                     if (!low) mma_bf16(Olo[mt], a0, a1, a2, a3, pl[0], pl[1]);
@@ -492,6 +566,14 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
                         for (int k = 0; k < 4; ++k) {
                             const uint2 a0 = lut_pairs<kLutStride>(lut, even[0], k), a1 = lut_pairs<kLutStride>(lut, odd[0], k);
                             const uint2 a2 = lut_pairs<kLutStride>(lut, even[1], k), a3 = lut_pairs<kLutStride>(lut, odd[1], k);
+                            if constexpr (EXACT) {
+                                uint4 a[3] = {make_uint4(a0.x, a1.x, a2.x, a3.x), make_uint4(a0.y, a1.y, a2.y, a3.y), make_uint4(0u, 0u, 0u, 0u)};
+                                if (two_terms)
+                                    a[2] = make_uint4(lut_third<kLut2Stride>(lut2, even[0], k), lut_third<kLut2Stride>(lut2, odd[0], k),
+                                                      lut_third<kLut2Stride>(lut2, even[1], k), lut_third<kLut2Stride>(lut2, odd[1], k));
+                                pv_exact(4 * b + k, a, two_terms ? 3 : 1);
+                                continue;
+                            }
                             pv(4 * b + k, a0.x, a1.x, a2.x, a3.x, false);
                             if (two_terms) pv(4 * b + k, a0.y, a1.y, a2.y, a3.y, true);
                         }
@@ -517,6 +599,8 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
                 const float hi_sum = O[mt][i];
                 float lo_sum;
                 if constexpr (G == 8) lo_sum = Olo[mt][i];
+                else if constexpr (EXACT && G == 2) lo_sum = __shfl_down_sync(0xffffffffu, hi_sum, 1) + __shfl_down_sync(0xffffffffu, hi_sum, 2);
+                else if constexpr (EXACT && G == 1) lo_sum = __shfl_down_sync(0xffffffffu, hi_sum, 1) + O[mt][i | 1];
                 else lo_sum = __shfl_xor_sync(0xffffffffu, hi_sum, 2);  // columns 4..7 are the low parts of heads 0..3
                 const int hd = 2 * j + (i & 1);
                 int d;  // element that row g (i < 2) or g + 8 of m-tile mt stands for
@@ -550,11 +634,11 @@ decode_mma_kernel(ViewDev view, const uint16_t *__restrict__ q, const int32_t *_
     mm_wait<0>();
 }
 
-template <int KIND, int D, int G>
+template <int KIND, int D, int G, bool EXACT>
 static int32_t launch_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
                           float *lse_part, int *err, int max_ctas, int *n_ctas_out, bool after_write, const AppendArgs &ap, cudaStream_t s) {
-    using LT = MmLayout<KIND, D, G>;
-    auto kern = decode_mma_kernel<KIND, D, G>;
+    using LT = MmLayout<KIND, D, G, EXACT>;
+    auto kern = decode_mma_kernel<KIND, D, G, EXACT>;
     static PerDeviceState configured;
     const int dev = current_device();
     if (configured.get(dev) == 0) {
@@ -584,11 +668,13 @@ static int32_t launch_mma(const ViewDev &v, const uint16_t *q, const int32_t *se
 }
 
 // `ap` (a bf16 cache of one sequence in one page, else k_new == NULL): the step's new token.  *n_ctas_out = CTAs per kv head, *tile_out = tokens per tile, as the merge kernel needs them.
+// `exact`: the caller takes fp32 results.
 int32_t decode_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads, float scale_log2, float *o_part,
-                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, const AppendArgs &ap, cudaStream_t s) {
+                   float *lse_part, int *err, int max_ctas, int *n_ctas_out, int *tile_out, bool after_write, bool exact, const AppendArgs &ap, cudaStream_t s) {
     *tile_out = kMmTile;
     const int G = n_q_heads / v.n_kv_heads;
-#define HS_MMA_RUN(K, DD, GG) launch_mma<K, DD, GG>(v, q, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, max_ctas, n_ctas_out, after_write, ap, s)
+#define HS_MMA_ARGS v, q, seq_lens, n_seqs, n_q_heads, scale_log2, o_part, lse_part, err, max_ctas, n_ctas_out, after_write, ap, s
+#define HS_MMA_RUN(K, DD, GG) exact ? launch_mma<K, DD, GG, true>(HS_MMA_ARGS) : launch_mma<K, DD, GG, false>(HS_MMA_ARGS)
 #define HS_MMA_G(K, DD) \
     switch (G) { \
         case 1: return HS_MMA_RUN(K, DD, 1); \
@@ -612,6 +698,7 @@ int32_t decode_mma(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens,
 #undef HS_MMA_D
 #undef HS_MMA_G
 #undef HS_MMA_RUN
+#undef HS_MMA_ARGS
 }
 
 }  // namespace hs

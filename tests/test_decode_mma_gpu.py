@@ -30,7 +30,7 @@ def _stored(t, kind, block, sdt):
     return (book[idx].view(-1, block) * torch.from_numpy(amax.astype("float64"))[:, None]).view(t.shape)
 
 
-def _run(cuda, hq, hkv, d, lens, page_tokens, seed, edit=None, kind=0, block=64, sdt=0):
+def _run(cuda, hq, hkv, d, lens, page_tokens, seed, edit=None, kind=0, block=64, sdt=0, shard=False):
     from hyprstream_b200 import kv_cache as kc
     from hyprstream_b200 import ops
 
@@ -49,9 +49,9 @@ def _run(cuda, hq, hkv, d, lens, page_tokens, seed, edit=None, kind=0, block=64,
         kvs.append((k[0], v[0]) if kind == 0 else tuple(_stored(t, kind, block, sdt) for t in (k[0], v[0])))
     q = torch.randn(len(lens), hq, d, generator=g).bfloat16()
     view, keep = kc.make_view(caches)
-    out = ops.decode_attention(q.to(cuda), view, torch.tensor(lens, dtype=torch.int32, device=cuda))
+    out = ops.decode_attention(q.to(cuda), view, torch.tensor(lens, dtype=torch.int32, device=cuda), shard=shard)
     torch.cuda.synchronize()
-    return q, kvs, out.cpu()
+    return q, kvs, tuple(t.cpu() for t in out) if shard else out.cpu()
 
 
 @pytest.mark.parametrize("d", [64, 128, 256])
@@ -294,3 +294,20 @@ def test_nf4_decode_infinite_value(cuda, d, g):
     assert (o[0, :, 5] == -math.inf).all() and (o[1, :, d - 1] == -math.inf).all()
     assert o[0, :, :64].isnan().sum().item() == o[1, :, d - 64:].isnan().sum().item() == 63 * g
     assert torch.isfinite(o).sum().item() == o.numel() - 2 * 64 * g
+
+
+@pytest.mark.parametrize("kind,d,block", [(0, 64, 64), (0, 128, 64), (0, 256, 64), (1, 64, 64), (1, 128, 128), (1, 256, 256), (2, 64, 64), (2, 128, 128),
+                                          (2, 256, 64), (3, 128, 64)])
+@pytest.mark.parametrize("g", [1, 2, 4, 8])
+def test_shard_results_in_fp32(cuda, kind, d, block, g):
+    """fp32 results (a KV-length shard's output and log-sum-exp) are as near to 64 bits as fp32 weights and table values make them.  A
+    score of up to 16 (in powers of two) is rounded to 2^-21, exp2f is good to 2 ulp (2^-22): 7e-7 of a weight at worst, 5e-7 of the
+    natural logarithm, and one fp32 rounding of a log-sum-exp below 16 on top (5e-7)."""
+    lens = [1, 17, 333, 3000]
+    q, kvs, (o, lse) = _run(cuda, 2 * g, 2, d, lens, 0, seed=d + g, kind=kind, block=block, shard=True)
+    for r, (k, v) in enumerate(kvs):
+        ref = _attend64(q[r], k, v)
+        s = torch.einsum("hd,lhd->hl", q[r].double(), k.double().repeat_interleave(g, 1)) / math.sqrt(d)
+        assert (o[r].double() - ref).norm() <= 7e-7 * ref.norm(), (lens[r], ((o[r].double() - ref).norm() / ref.norm()).item())
+        assert (lse[r].double() - s.logsumexp(-1)).abs().max() <= 1.2e-6, lens[r]
+
