@@ -10,8 +10,6 @@
 //
 // This file is host code: it chains the library's own entry points and only carves their intermediates out of the
 // caller's workspace.
-#include <vector>
-
 #include "hs_common.cuh"
 
 namespace hs {
@@ -35,22 +33,35 @@ static GdnScratch gdn_scratch(const hs_gdn_layer_params *p, int64_t n_seqs, int6
     return s;
 }
 
-// Address ranges that the kernels of a block read (or also write).
+// Address ranges that the kernels of one layer's decode step read (or also write).  A fixed array: nothing here may throw.
 struct Spans {
     struct Span { uintptr_t b, e; bool written; };
-    std::vector<Span> v;
+    Span v[8];
+    int n = 0;
     void add(const void *p, int64_t bytes, bool written) {
         const uintptr_t b = reinterpret_cast<uintptr_t>(p);
-        v.push_back({b, b + static_cast<uintptr_t>(bytes > 0 ? bytes : 0), written});
+        v[n++] = {b, b + static_cast<uintptr_t>(bytes > 0 ? bytes : 0), written};
     }
-    // nothing from index `first` on touches what the ranges before it write, or writes what they touch
-    bool apart(size_t first) const {
-        for (size_t i = first; i < v.size(); ++i)
-            for (size_t j = 0; j < first; ++j)
-                if ((v[i].written || v[j].written) && v[i].b < v[j].e && v[j].b < v[i].e) return false;
+    // neither layer touches what the other writes
+    bool apart(const Spans &o) const {
+        for (int i = 0; i < n; ++i)
+            for (int j = 0; j < o.n; ++j)
+                if ((v[i].written || o.v[j].written) && v[i].b < o.v[j].e && o.v[j].b < v[i].e) return false;
         return true;
     }
 };
+static Spans gdn_step_spans(const hs_gdn_layer_params &p, const hs_gdn_layer_io &io, int64_t n) {
+    const int64_t vd = static_cast<int64_t>(p.n_v_heads) * p.head_v_dim, conv = 2LL * p.n_k_heads * p.head_k_dim + vd;
+    Spans s;
+    s.add(io.mixed_qkv, n * conv * 2, false);
+    s.add(io.z, n * vd * 2, false);
+    s.add(io.a_in, n * p.n_v_heads * 2, false);
+    s.add(io.b_in, n * p.n_v_heads * 2, false);
+    s.add(io.conv_state, n * conv * (p.kernel_size - 1) * 2, true);
+    s.add(io.rec_state, n * vd * p.head_k_dim * 4, true);
+    s.add(io.y, n * vd * 2, true);
+    return s;
+}
 
 static int32_t check_gdn_params(const hs_gdn_layer_params *p, const char *who) {
     if (!p) return fail(HS_ERR_ARG, "%s: NULL layer parameters", who);
@@ -207,39 +218,31 @@ int32_t hs_qwen_block_forward(const hs_gdn_layer_params *gdn, const hs_gdn_layer
     if ((attn == nullptr) != (attn_io == nullptr)) return fail(HS_ERR_ARG, "hs_qwen_block_forward: attention parameters and inputs go together");
     // A decode step's layers read only what the caller has handed in, so each kernel may start beside the one before it - unless
     // buffers are shared between layers: every layer's inputs, states and outputs are compared with those of the layers before.
-    Spans spans;
+    const bool may_overlap = n_tokens == 1 && has_state && n_seqs > 0;
+    auto apart_from = [&](const Spans &mine, int layers) {  // ... from the first `layers` DeltaNet layers
+        for (int j = 0; j < layers; ++j)
+            if (!mine.apart(gdn_step_spans(gdn[j], gdn_io[j], n_seqs))) return false;
+        return true;
+    };
     for (int i = 0; i < n_gdn; ++i) {
         const hs_gdn_layer_io &io = gdn_io[i];
-        bool overlap = false;
-        if (n_tokens == 1 && has_state && n_seqs > 0) {
-            const hs_gdn_layer_params &p = gdn[i];
-            const int64_t n = n_seqs, vd = static_cast<int64_t>(p.n_v_heads) * p.head_v_dim, conv = 2LL * p.n_k_heads * p.head_k_dim + vd;
-            const size_t first = spans.v.size();
-            spans.add(io.mixed_qkv, n * conv * 2, false);
-            spans.add(io.z, n * vd * 2, false);
-            spans.add(io.a_in, n * p.n_v_heads * 2, false);
-            spans.add(io.b_in, n * p.n_v_heads * 2, false);
-            spans.add(io.conv_state, n * conv * (p.kernel_size - 1) * 2, true);
-            spans.add(io.rec_state, n * vd * p.head_k_dim * 4, true);
-            spans.add(io.y, n * vd * 2, true);
-            overlap = i > 0 && spans.apart(first);
-        }
+        const bool overlap = may_overlap && i > 0 && apart_from(gdn_step_spans(gdn[i], io, n_seqs), i);
         if (int32_t st = gdn_layer_forward_impl(gdn + i, io.mixed_qkv, io.z, io.a_in, io.b_in, io.conv_state, io.rec_state, has_state, n_seqs, n_tokens, io.y,
                                                 workspace, workspace_bytes, overlap, stream))
             return st;
     }
     if (attn) {
         bool overlap = false;
-        if (n_tokens == 1 && has_state && n_seqs > 0 && n_gdn > 0) {
+        if (may_overlap && n_gdn > 0) {
             const int64_t n = n_seqs, d = attn->head_dim;
-            const size_t first = spans.v.size();
-            spans.add(attn_io->q_proj, n * attn->n_q_heads * 2 * d * 2, false);
-            spans.add(attn_io->k_proj, n * attn->n_kv_heads * d * 2, false);
-            spans.add(attn_io->v_proj, n * attn->n_kv_heads * d * 2, false);
-            spans.add(attn_io->positions, n * 4, false);
-            spans.add(attn_io->dst_pos, n * 4, false);
-            spans.add(workspace, workspace_bytes, true);
-            overlap = spans.apart(first);
+            Spans s;
+            s.add(attn_io->q_proj, n * attn->n_q_heads * 2 * d * 2, false);
+            s.add(attn_io->k_proj, n * attn->n_kv_heads * d * 2, false);
+            s.add(attn_io->v_proj, n * attn->n_kv_heads * d * 2, false);
+            s.add(attn_io->positions, n * 4, false);
+            s.add(attn_io->dst_pos, n * 4, false);
+            s.add(workspace, workspace_bytes, true);
+            overlap = apart_from(s, n_gdn);
         }
         return attn_layer_forward_impl(attn, attn_io->q_proj, attn_io->k_proj, attn_io->v_proj, attn_io->view, attn_io->positions, attn_io->dst_pos,
                                        attn_io->seq_lens, n_seqs, n_tokens, attn_io->out, workspace, workspace_bytes, overlap, stream);
