@@ -142,7 +142,7 @@ __global__ void merge_parts_kernel(const float *__restrict__ o_parts, const floa
 static int decode_max_ctas() { return 4 * sm_count(); }
 constexpr int kMaxPartsPerPair = 2;
 
-// decode_tc.cu: tensor-core kernel for the int8 / head_dim 128 / 8 kv heads / group 4 shape
+// decode_tc.cu: cooperative tensor-core kernel for the quantised caches of the two served models' shapes
 int32_t decode_int8_tc_try(const ViewDev &v, const uint16_t *q, const int32_t *seq_lens, int n_seqs, int n_q_heads,
                            float softmax_scale, float *o_part, float *lse_part, int *err, cudaStream_t s, int *n_ctas_out,
                            uint16_t *out, const uint16_t *gate, float *o_shard, float *lse_shard, int *merged_out,
@@ -377,8 +377,8 @@ int32_t hs_attn_decode_step(const hs_kv_view *view, const void *host_in, void *d
     cudaError_t e = cudaMemcpyAsync(dev_in, host_in, static_cast<size_t>(q_elems + 2 * kv_elems) * 2, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(static_cast<int32_t>(e), "hs_attn_decode_step: %s", cudaGetErrorString(e));
     uint16_t *qd = reinterpret_cast<uint16_t *>(dev_in), *kd = qd + q_elems, *vd = kd + kv_elems;
-    // cache update + attention: one launch when the new tokens go to seq_lens - 1 (dst_pos == NULL) on a u8 cache, else the write
-    // kernel and the attention kernel as its programmatic dependent; q came with the copy before both
+    // cache update + attention: where the attention kernel writes the tokens itself one launch less (see above), else the write kernel
+    // and the attention kernel as its programmatic dependent; q came with the copy before both
     if (int32_t st = hs_attn_decode_append(qd, kd, vd, view, dst_pos, seq_lens, n_seqs, n_q_heads, softmax_scale, sin, cos, rotary_dim, n_positions, dev_out,
                                            nullptr, workspace, workspace_bytes, stream))
         return st;

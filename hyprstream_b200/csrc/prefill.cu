@@ -222,7 +222,7 @@ static int32_t launch_prefill(const uint16_t *q, const uint16_t *k, const uint16
     return HS_OK;
 }
 
-// prefill_tc5.cu: tcgen05 / TMEM / TMA kernel for head_dim 128
+// prefill_tc5.cu: tcgen05 / TMEM / TMA kernels
 int32_t prefill_tc5_try(const uint16_t *q, const uint16_t *k, const uint16_t *v, uint16_t *out, const uint16_t *gate, int64_t gate_ts,
                         int64_t gate_hs, int n_seqs, int q_len, int kv_len, int n_q_heads, int n_kv_heads, int head_dim, float scale_log2,
                         cudaStream_t s, int *taken);

@@ -18,10 +18,17 @@
 // Why steps of 64 keys: with one 128-column score buffer per query tile a tile's softmax and its MMAs took turns (clock64 stamps,
 // 128 keys: softmax 1,820 cycles, hand-over 220, P.V + S 1,290 = 3,330 a round, tensor pipe and XU both half idle).  Two 64-column
 // buffers per query tile let S_{u+1} be ready when the softmax of step u ends: 2,720 cycles a round of 128 keys.  What bounds it
-// now: head_dim 128 the shared-memory reads of the 64-column S (A and B, 6 KB per 128 x 64 x 16 MMA: 320 KB a round against 128 B a
-// cycle; 128-column S with one buffer reads 256 KB but takes turns: 10 % slower), head_dim 64 the softmax warps (75 % of the XU).
+// now: head_dim 128 the shared-memory traffic, 320 KB a round against 128 B a cycle: S reads 192 KB (A and B, 6 KB per 128 x 64 x 16
+// MMA, 16 of them per tile), P.V 64 KB of V, and the K/V tiles are written with 64 KB (128-column S with one buffer: 128 + 64 + 64 KB,
+// but it takes turns: 10 % slower); head_dim 64 the softmax warps (75 % of the XU).
 // Measured against the one-buffer, one-issuer form (32 / 8 heads): 4 x 8,192 x 128 2.13 -> 1.94 ms = 1.13 PFLOP/s; 1,000 queries
 // behind 3,333 keys 73 -> 67 us; 100 behind 7,900 111 -> 89 us; head_dim 64: 8 x 4,096 1.03 -> 0.87 ms, 2 x 1,531 63 -> 55 us.
+//
+// P is rounded to bf16 relative to a row's reference maximum; a weight that equals the reference is exact (a power of two).  The
+// reference is taken over the first 64 keys and moved when the maximum has grown by 2^8, so the error against 64 bits is a little above
+// that of the forms that knew more keys first: head_dim 128, 1,531 keys 2.07e-3 -> 2.09e-3 (reference over 128 keys), head_dim 64
+// 2.01e-3 -> 2.07e-3 (the running maximum of the mma.sync kernel).  Taking it over the first two steps here gives the 2.07e-3 and
+// was measured 2 to 8 % slower (the first exponentials wait for both tiles' second S): 1,000 behind 3,333 keys 67 -> 72 us.
 //
 // TMEM columns: S/P of tile x and step u at 128 x + 64 (u & 1), O of tile x at 256 + D x.  Shared memory (D = 128): 2 x Q 32 KB
 // + 2 x (K 32 KB + V 32 KB).  FLOPs per (query tile, step): 2 x 2 x 128 x 64 x D.
@@ -906,16 +913,17 @@ static int32_t launch_t5(const uint16_t *q, const uint16_t *k, const uint16_t *v
     return HS_OK;
 }
 
-// Returns HS_OK with *taken = 1 when this kernel took the launch, *taken = 0 when the caller should use the
-// mma.sync kernel (a single query token, an output that is not
-// 16-byte aligned, or no tensor-map encoder in the driver).
+// Returns HS_OK with *taken = 1 when this kernel took the launch, *taken = 0 when the caller should use the mma.sync kernel (a single
+// query token, an output that is not 16-byte aligned, head_dim 64 with few keys, or no tensor-map encoder in the driver).
 int32_t prefill_tc5_try(const uint16_t *q, const uint16_t *k, const uint16_t *v, uint16_t *out, const uint16_t *gate, int64_t gate_ts,
                         int64_t gate_hs, int n_seqs, int q_len, int kv_len, int n_q_heads, int n_kv_heads, int head_dim, float scale_log2,
                         cudaStream_t s, int *taken) {
     *taken = 0;
     if (q_len < 2 || !aligned(out, 16)) return HS_OK;  // (the epilogue stores 16 bytes at a time)
-    // head_dim 64, all keys in one or two of the mma.sync kernel's tiles: its shorter start wins (32 heads: 4.7 against 6.7 us at 64 keys,
-    // 6.4 against 7.0 at 128, 10.0 against 10.1 at 256; 31.2 against 13.8 at 600)
+    // head_dim 64, up to three of the mma.sync kernel's 64-key tiles: its shorter start and 64-row blocks.  Whole calls, 32 heads, mma.sync
+    // against this kernel: one prompt of 193 keys 10.6 / 10.0 us, of 256 12.0 / 9.9; 8 of 128 13.7 / 14.4, of 160 22.0 / 16.5; 32 of 64
+    // 16.5 / 32.8, of 128 34.8 / 41.0, of 192 59.4 / 49.2.  So the two cross near 192 keys, where the line is, with one prompt, and
+    // between 128 and 160 with several.
     if (head_dim == 64 && kv_len <= 192) return HS_OK;
     if (head_dim == kW5D) {
         CUtensorMap mq, mk, mv;

@@ -126,8 +126,8 @@ def test_pages_aligned_to_words(cuda, kind, d, g, shift):
 @pytest.mark.parametrize("hq,hkv,d,rotary", [(32, 8, 128, 128), (4, 2, 64, 64), (16, 2, 256, 64), (3, 3, 128, 0)])
 @pytest.mark.parametrize("page_tokens", [0, 40, 256])
 def test_bf16_step_writes_its_token(cuda, hq, hkv, d, rotary, page_tokens):
-    """decode_append without positions (the attention kernel writes the new token of every sequence) leaves the same cache and gives
-    the same output as the write kernel followed by the attention, bit for bit - also where the rotation table ends."""
+    """decode_append without positions (a batch: the tokens are written first, at seq_lens - 1) leaves the same cache and gives the same
+    output as with positions, bit for bit - also where the rotation table ends."""
     from hyprstream_b200 import ffi, kv_cache as kc, ops
 
     lens = [1, 2, 16, 17, 32, 40, 41, 639]

@@ -76,8 +76,8 @@ def test_static_scratch_decode_matches_workspace_decode_twice(cuda):
 
 
 def test_static_scratch_serves_the_generic_kernel_and_its_merge_too(cuda):
-    """A shape the tensor-core kernel does not cover (4 q / 2 kv heads, head_dim 64): the CUDA-core decode kernel and
-    the separate merge kernel both run out of the built-in array; two calls in a row, no allocation."""
+    """A shape the cooperative kernel does not cover (4 q / 2 kv heads, head_dim 64): the general decode kernel and the
+    separate merge kernel both run out of the built-in array; two calls in a row, no allocation."""
     from hyprstream_b200 import ffi, kv_cache as kc, ops
 
     lens = [300, 5, 1025]
