@@ -340,6 +340,7 @@ int32_t hs_attn_decode_append(const void *q, const void *k_new, const void *v_ne
         // batch may look at one another's new tokens, several tokens of one sequence handed in as rows, and a table may list a page
         // twice: the host cannot see either, so everything that could is written before anything is attended.  One launch against
         // two: 1 x 4,096 tokens 34.3 against 36.0 us, 16 paged sequences 53.9 against 55.4 us.)
+        if (!seq_lens && n_seqs > 0) return fail(HS_ERR_ARG, "hs_attn_decode_append: NULL lengths");  // (before anything is written)
         if (!aligned(k_new, 16) || !aligned(v_new, 16)) return fail(HS_ERR_ARG, "hs_attn_decode_append: inputs must be 16-byte aligned");
         if (sin != nullptr && (!cos || rotary_dim <= 0 || rotary_dim % 16 != 0 || (view && rotary_dim > view->head_dim) || n_positions <= 0))
             return fail(HS_ERR_UNSUPPORTED, "hs_attn_decode_append: rotary_dim must be a positive multiple of 16 <= head_dim");

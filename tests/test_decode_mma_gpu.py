@@ -1,5 +1,6 @@
 """GPU: the tensor-core decode kernel for every kind, head_dim, scale block and query group it serves, at the edges of its 16-token
 tiles, of its CTA ranges and of pages that are no multiple of a tile; and code pages that are aligned to words only."""
+import ctypes
 import math
 
 import pytest
@@ -311,3 +312,24 @@ def test_shard_results_in_fp32(cuda, kind, d, block, g):
         assert (o[r].double() - ref).norm() <= 7e-7 * ref.norm(), (lens[r], ((o[r].double() - ref).norm() / ref.norm()).item())
         assert (lse[r].double() - s.logsumexp(-1)).abs().max() <= 1.2e-6, lens[r]
 
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_append_without_lengths_is_refused_untouched(cuda, kind):
+    """Neither positions nor lengths: refused, the cache as it was and no device error left behind."""
+    from hyprstream_b200 import ffi, kv_cache as kc, ops
+
+    g = torch.Generator().manual_seed(kind)
+    kv = [torch.randn(1, 20, 2, 64, generator=g).bfloat16().to(cuda) for _ in range(2)]
+    caches = [kc.LayerKVCache(64, kc.KVQuantType(kind), 2, 64, cuda) for _ in range(2)]
+    for c in caches:
+        c.update(*kv, 0)
+    before = [t.clone() for c in caches for t in c.get()]
+    view, keep = kc.make_view(caches)
+    x = torch.ones(2, 4, 64, dtype=torch.bfloat16, device=cuda)
+    ws = ops.decode_workspace(2, 4, 64, cuda)
+    st = ffi.lib.hs_attn_decode_append(x.data_ptr(), x.data_ptr(), x.data_ptr(), ctypes.byref(view), None, None, 2, 4, ctypes.c_float(0.125), None, None, 0, 0,
+                                       torch.empty_like(x).data_ptr(), None, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert st == ffi.HS_ERR_ARG
+    torch.cuda.synchronize()
+    assert ffi.take_device_error() == 0
+    assert all(torch.equal(a, b) for a, b in zip(before, [t for c in caches for t in c.get()]))
